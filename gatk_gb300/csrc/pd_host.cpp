@@ -272,16 +272,35 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s) 
     GHMM_CUDA(cudaEventRecord(b.ev[1], s), "event");
     int launches = 0;
     if (packed) {  // read-pair tasks, then the log10 epilogue of their sums (before the kernels that write log10)
+        // captured once and replayed while the batch's pointers and buckets stay the same, as the regular forward is
+        std::vector<unsigned char> sig(sizeof(DevBatch) + sizeof(PdPlanes));
+        memcpy(sig.data(), &b.dev, sizeof(DevBatch));
+        memcpy(sig.data() + sizeof(DevBatch), &b.pd, sizeof(PdPlanes));
         for (auto &bk : b.buckets) {
-            int bp = 0;
-            if (pd_bucket_occupancy(bk.key, &bp) != 0 || bp <= 0) bp = 1;
-            const int64_t want = (bk.count + kWarpsPerBlock - 1) / kWarpsPerBlock;
-            int g = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * bp));
-            if (bk.key & 16) g = std::min(g, bk.grid);  // the strip scratch is sized for the regular kernel's grid
-            int e = launch_pd_bucket(ctx->tables, b.dev, b.pd.ops, bk.key, g, s);
-            if (e) return cuda_fail(ctx, (cudaError_t)e, "PD-HMM packed launch");
-            launches++;
+            const int kg[3] = {bk.key, bk.grid, bk.count};
+            const unsigned char *k3 = (const unsigned char *)kg;
+            sig.insert(sig.end(), k3, k3 + sizeof(kg));
         }
+        if (sig != b.graph_sig) {
+            if (b.graph[0]) cudaGraphExecDestroy(b.graph[0]);
+            b.graph[0] = nullptr;
+            b.graph_sig.clear();
+            const int rc = capture_graph(ctx, s, &b.graph[0], [&] {
+                return fork_buckets(ctx, b, s, [&](const Bucket &bk, const DevBatch &d, cudaStream_t st) {
+                    int bp = 0;
+                    if (pd_bucket_occupancy(bk.key, &bp) != 0 || bp <= 0) bp = 1;
+                    const int64_t want = (bk.count + kWarpsPerBlock - 1) / kWarpsPerBlock;
+                    int g = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * bp));
+                    if (bk.key & 16) g = std::min(g, bk.grid);  // the strip scratch is sized for the regular kernel's grid
+                    const int e = launch_pd_bucket(ctx->tables, d, b.pd.ops, bk.key, g, st);
+                    return e ? cuda_fail(ctx, (cudaError_t)e, "PD-HMM packed launch") : GHMM_OK;
+                });
+            });
+            if (rc) return rc;
+            b.graph_sig = sig;
+        }
+        GHMM_CUDA(cudaGraphLaunch(b.graph[0], s), "graph launch");
+        launches += (int)b.buckets.size();
         int e = launch_finalize_fp32(b.dev.out, b.dev.n_out_dev, ctx->sm_count, s);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "PD-HMM FP32 finalize launch");
         launches++;

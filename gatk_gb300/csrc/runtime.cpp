@@ -265,6 +265,10 @@ int ghmm_done(ghmm_ctx *ctx) {
         if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->pd_stream2) cudaStreamDestroy(ctx->pd_stream2);
+    for (auto &st : ctx->fork_stream)
+        if (st) cudaStreamDestroy(st);
+    for (auto &ev : ctx->fork_ev)
+        if (ev) cudaEventDestroy(ev);
     delete ctx;
     return GHMM_OK;
 }

@@ -11,6 +11,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <deque>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -35,7 +36,10 @@ struct Bucket {
     int key;  // rows-per-lane | 16 if multi-strip
     int begin, count;
     int grid;
+    int scratch_block;  // multi-strip buckets run side by side: first block of this bucket's part of the strip scratch
 };
+// The most kernels of one forward that run side by side: the caller's stream and kForkStreams forked from it.
+constexpr int kForkStreams = 4;
 
 // Routing of reads whose gap penalties are only known after the device imputation (DRAGstr).  The checks that
 // guard against wrong finite results (a continuation penalty of 0, a matchToMatch probability of about 0) are
@@ -114,6 +118,7 @@ struct ghmm_batch {
     int64_t n_direct_fp64mode = 0, n_fp64mode_exact = 0;
     std::vector<uint8_t> read_exact;  // reads whose pairs go to the exact FP64 tier directly
     int64_t scratch32_cols = 0;
+    int scratch32_blocks = 0;
     int fp64_grid = 0;
     // last forward
     int last_mode = -1;
@@ -130,7 +135,7 @@ struct ghmm_batch {
     bool prep_events = false, prep_timed = false;
     int64_t pending_n_pre = 0;
     int pending_mode = -1;
-    cudaGraphExec_t graph[2]{};  // captured FP32 phase and FP64 phase
+    cudaGraphExec_t graph[2]{};  // captured FP32 phase (PD batches: its packed buckets) and FP64 phase
     std::vector<unsigned char> graph_sig;  // DevBatch bytes, mode, bucket keys and grids the graphs were captured for
 
     void release() {
@@ -183,6 +188,11 @@ struct ghmm_ctx {
     DevBuf<uint8_t> calib_scratch;
     DevBuf<int> calib_flags;
     DevBuf<double> calib_ones;
+    // streams a captured forward forks its bucket kernels onto; used only while capturing, under fork_mu (the queue's
+    // worker and the caller's thread may both capture)
+    cudaStream_t fork_stream[kForkStreams]{};
+    cudaEvent_t fork_ev[kForkStreams + 1]{};
+    std::mutex fork_mu;
     ghmm_queue *pipe = nullptr;      // the queue that pipelines large synchronous calls
     std::atomic<int> open_queues{0};  // queues of this context not yet destroyed (including pipe)
     SwEngine *sw = nullptr;          // Smith-Waterman buffers (sw_host.cpp), created on first use
@@ -295,6 +305,9 @@ int batch_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s);
 int fill_fp64_all(ghmm_ctx *ctx, ghmm_batch &b);
 int batch_forward(ghmm_ctx *ctx, ghmm_batch &b, int mode);
 int batch_enqueue(ghmm_ctx *ctx, ghmm_batch &b, int mode, cudaStream_t s);
+int capture_graph(ghmm_ctx *ctx, cudaStream_t s, cudaGraphExec_t *out, const std::function<int()> &enqueue);
+int fork_buckets(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s, const std::function<int(const Bucket &, const DevBatch &, cudaStream_t)> &launch);
+int64_t task_cols(int64_t pair_cols, int sm_count, int64_t max_cols);  // haplotype columns per FP32 task
 int batch_finish(ghmm_ctx *ctx, ghmm_batch &b);
 int batch_results(ghmm_ctx *ctx, ghmm_batch &b, double *out);
 int batch_results_on(ghmm_ctx *ctx, ghmm_batch &b, double *out, cudaStream_t s);
