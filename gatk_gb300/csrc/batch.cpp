@@ -464,7 +464,7 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
     }
     b.scratch32_cols = max_multi_cols;
     int bpsm64 = 0;
-    if (fp64_kernel_occupancy(kBlock, &bpsm64) != 0 || bpsm64 <= 0) bpsm64 = 1;
+    if (fp64_kernel_occupancy(&bpsm64) != 0 || bpsm64 <= 0) bpsm64 = 1;
     b.fp64_grid = ctx->sm_count * bpsm64;
     b.uploaded = false;
     const auto t_end = std::chrono::steady_clock::now();
@@ -630,7 +630,7 @@ int batch_phase(ghmm_ctx *ctx, ghmm_batch &b, int phase, cudaStream_t s) {
         }
         return GHMM_OK;
     }
-    int e = launch_fp64_queue(ctx->tables, b.dev, b.fp64_grid, kBlock, s);
+    int e = launch_fp64_queue(ctx->tables, b.dev, b.max_read_len >= kFp64SplitRows, b.fp64_grid, s);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "FP64 queue launch");
     return GHMM_OK;
 }
@@ -737,6 +737,8 @@ int batch_enqueue(ghmm_ctx *ctx, ghmm_batch &b, int mode, cudaStream_t s) {
     memcpy(sig.data() + sizeof(DevBatch), &mode, sizeof(int));
     const int has_tasks = b.n_tasks > 0;
     memcpy(sig.data() + sizeof(DevBatch) + sizeof(int), &has_tasks, sizeof(int));
+    const int fp64_args[2] = {b.max_read_len >= kFp64SplitRows, b.fp64_grid};
+    sig.insert(sig.end(), (const unsigned char *)fp64_args, (const unsigned char *)fp64_args + sizeof(fp64_args));
     for (auto &bk : b.buckets) {
         const int kg[2] = {bk.key, bk.grid};
         const unsigned char *k = (const unsigned char *)kg;

@@ -1,0 +1,406 @@
+// fp64.cu -- the FP64 wavefront: reruns of FP32 underflows, pairs routed to FP64, and double-precision mode, in two
+// tiers of one kernel template.  (Recurrence and citations: kernels.cu.)
+//
+// RESCALED (queue 1: host-routed pairs and FP32 underflows): the FP32 kernel's rescaled recurrence in FP64,
+// 5 DP operations per cell instead of 8 (the FP64 pipe runs at 1/64 of the FP32 rate on this part):
+//    M~ = prior * fma(I~_diag, b_i, fma(D~_diag, c_i, M~_diag)),  I~ = fma(I~_up, e_i, M~_up),
+//    D~ = fma(D~_left, DD_i, M~_left),  sum over the haplotype of M~_R + (MI_R / MM_R) I~_R.
+// The scale is S' = 2^960 instead of 2^1020 (headroom for I~ and D~, which carry 1 / MI and 1 / MD), and the
+// initial condition is divided by 2^round(la), la = log2 a_R = sum of -log2 MM_i, so that the last row sits at
+// scale S' like the unscaled recurrence.  Along every contributing path the rescaled states stay above the
+// final sum's magnitude, so a result of log10 L >= kRescaledFloor (well inside the FP64 range at S') is as
+// accurate as the unscaled recurrence; lower or non-finite results go to queue 2.
+//
+// EXACT (queue 2: those, and reads the host marks, e.g. matchToMatch ~ 0): the unscaled recurrence with the
+// reference's 2^1020 initial condition, so it underflows exactly where LoglessPairHMM does.
+//
+// What bounds it: the FP64 pipe, and that pipe is one per SM sub-partition: a warp's DFMA takes 64 cycles whether or
+// not the other three sub-partitions work (register loop: 0.156 Tops/s with one warp per SM at any instruction-level
+// parallelism, 0.625 with four).  Hence:
+//  * Everything but DP operations is free (64 issue slots per DP operation), and every DP operation counts.  A DMUL or
+//    DADD costs 19 cycles an SM where a DFMA costs 16, also a DFMA that the compiler can turn into one, so products
+//    and sums are DFMAs with a zero (or one) that only run time knows: the same roundings.  The last row is summed by
+//    all lanes once per 16 columns instead of by one lane in every column (two of 22 DP operations a step before).
+//  * Padding is work: a read's rows are split into strips of 32, 64, 96 or 128 rows that cover ceil(R / 32) * 32 rows
+//    instead of whole strips of 128 (reads of 100-250 bases: 191 rows on average instead of 232).
+//  * A pair on one warp uses a quarter of one SM.  Jobs are therefore either a pair per warp, its strips one after the
+//    other, or a pair per block: the strips go round the block's four warps, each strip 48 columns behind the one above
+//    it, in lockstep phases of 16 columns.
+// Measured against one pair per warp in strips of 128 rows (one GB300): 537 reads of 800-2,000 bases x haplotypes of
+// 1,500-3,000 (1.6e10 cells) 214 -> 158 ms, 103 of at most 125 GCUPS; 37,978 pairs of 100-250 bases (2.6e9 cells) all in
+// FP64 36.3 -> 27.2 ms; the 5 reruns of a region of 2,000 reads 0.85 -> 0.34 ms; 48 reruns of 260-600 bases x 800
+// 3.6 -> 1.1 ms.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "../../include/ghmm.h"
+#include "ghmm_internal.h"
+#include "warp_list.cuh"
+
+namespace ghmm {
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kWarps64 = 4;    // warps per block
+constexpr int kPhase = 16;     // columns (steps) of one phase
+constexpr int kStripLag = 3;   // phases a strip stays behind the strip above it: column c of the row above is written at
+                               // that strip's step c + 31, i.e. by the end of phase c / 16 + 2 at the latest
+constexpr double kLog10Scale64R = 288.9887958374219;   // log10(2^960)
+constexpr double kLog10Scale64 = 307.0505955772608;    // log10(2^1020)
+constexpr double kRescaledFloor = GHMM_FP64_RESCALED_FLOOR;
+
+// x * y and x + y at the DFMA rate; zero and one are kernel arguments, unknown to the compiler.  Every product here is
+// >= 0, so adding zero keeps its bits.
+struct Unit {
+    double zero, one;
+};
+__device__ __forceinline__ double mul64(double x, double y, Unit u) { return fma(x, y, u.zero); }
+__device__ __forceinline__ double add64(double x, double y, Unit u) { return fma(x, u.one, y); }
+
+// The pair of a job.
+struct Pair64 {
+    int64_t roff, out_index;
+    const uint8_t *hb;
+    int read, hap, R, H;
+    int blocks32;  // rows / 32, rounded up: the rows of all strips
+    int pad;       // dummy rows on top of strip 0 (0..31); they hold the row-0 boundary
+    double init, la;
+};
+
+__device__ __forceinline__ Pair64 load_pair(const DevBatch &B, PairRef pr) {
+    Pair64 P;
+    P.read = pr.read;
+    P.hap = pr.hap;
+    P.roff = B.read_off[pr.read];
+    P.R = (int)(B.read_off[pr.read + 1] - P.roff);
+    const int64_t hoff = B.hap_off[pr.hap];
+    P.H = (int)(B.hap_off[pr.hap + 1] - hoff);
+    P.hb = B.hap_bases + hoff;
+    const int region = B.read_region[pr.read];
+    const int64_t nh = B.region_hap_off[region + 1] - B.region_hap_off[region];
+    P.out_index = B.out_off[region] + (int64_t)(pr.read - B.region_read_off[region]) * nh +
+                  (pr.hap - B.region_hap_off[region]);
+    P.blocks32 = (P.R + 31) / 32;
+    P.pad = P.blocks32 * 32 - P.R;
+    P.la = 0.0;
+    P.init = 0.0;
+    return P;
+}
+
+// One strip of K <= 4 rows per lane: coefficients and running states of this lane's rows.
+template <bool RESCALED>
+struct Strip64 {
+    double pm[4], pe[4];
+    double c1[4], c2[4], c3[4], c4[4];  // RESCALED: b, c, e, unused; exact: MM, IM, MI, II
+    double c5[4];                       // exact: MD
+    double dd[4];                       // DD (1 in dummy rows, whose D stays at the row-0 value)
+    double M[4], I[4], D[4];
+    uint32_t base[4];
+    double gM, gI, gD;     // row above the lane's first row, previous column
+    double nxM, nxI, nxD;  // lane 0 below the first strip: the row above at the next column
+    int row0, k;           // first row (slot) of the strip, rows per lane
+    bool first, last;
+};
+
+// Strip `strip` of n strips that share the pair's 32-row blocks as evenly as they go, the larger ones first.
+template <bool RESCALED>
+__device__ __forceinline__ void strip_begin(const DevTables &T, const DevBatch &B, const Pair64 &P, int strip, int n,
+                                            const double *above, Strip64<RESCALED> &S, int lane) {
+    const int even = P.blocks32 / n, more = P.blocks32 - even * n;
+    S.k = even + (strip < more ? 1 : 0);
+    S.row0 = 32 * (strip * even + min(strip, more));
+    S.first = strip == 0;
+    S.last = strip == n - 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int p = S.row0 + lane * S.k + k - P.pad;
+        S.pm[k] = S.pe[k] = S.c1[k] = S.c2[k] = S.c3[k] = S.c4[k] = S.c5[k] = 0.0;
+        S.dd[k] = 1.0;
+        S.base[k] = 0x100u;  // matches nothing
+        if (k < S.k && p >= 0) {
+            const uint8_t base = B.bases[P.roff + p], q = B.quals[P.roff + p];
+            const uint8_t ins = B.ins[P.roff + p], del = B.dels[P.roff + p], gcp = B.gcp[P.roff + p];
+            S.pm[k] = __ldg(T.prob_d + q);
+            S.pe[k] = base == 'N' ? S.pm[k] : __ldg(T.err3_d + q);
+            S.base[k] = base;
+            const double mm = __ldg(T.m2m_d + ins * 128 + del), im = __ldg(T.prob_d + gcp);
+            const double mi = __ldg(T.err_d + ins), ii = __ldg(T.err_d + gcp), md = __ldg(T.err_d + del);
+            S.dd[k] = ii;
+            if (RESCALED) {
+                double mm_p = 1.0, mi_p = 1.0, md_p = 1.0;
+                if (p > 0) {
+                    const uint8_t ins_p = B.ins[P.roff + p - 1], del_p = B.dels[P.roff + p - 1];
+                    mm_p = __ldg(T.m2m_d + ins_p * 128 + del_p);
+                    mi_p = __ldg(T.err_d + ins_p);
+                    md_p = __ldg(T.err_d + del_p);
+                }
+                S.c1[k] = im * mi_p / (mm * mm_p);
+                S.c2[k] = im * md_p / mm;
+                S.c3[k] = p > 0 ? ii * mi_p / (mi * mm_p) : 0.0;
+            } else {
+                S.c1[k] = mm;
+                S.c2[k] = im;
+                S.c3[k] = mi;
+                S.c4[k] = ii;
+                S.c5[k] = md;
+            }
+        }
+    }
+    if (!S.first && lane == 0) {
+        S.nxM = above[0];
+        S.nxI = above[1];
+        S.nxD = above[2];
+    }
+}
+
+// Steps [s0, s1) of a strip of K rows per lane: at step s lane l computes column s - l.  The last row of a strip goes
+// to `below` for the next strip; the pair's last row goes to rowM / rowI, 16 steps at a time.
+template <int K, bool RESCALED>
+__device__ __forceinline__ void strip_steps(const Pair64 &P, Strip64<RESCALED> &S, int s0, int s1, const double *above,
+                                            double *below, double *rowM, double *rowI, Unit u, int lane) {
+    for (int s = s0; s < s1; ++s) {
+        const int c = s - lane;
+        const bool valid = c >= 0 && c < P.H;
+        const uint32_t y = valid ? (uint32_t)__ldg(P.hb + c) : 0x200u;
+        const bool yn = (y == 'N');
+        if (c == 0) {  // column-0 boundary (lanes compute ahead of their first column)
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                S.M[k] = S.I[k] = 0.0;
+                S.D[k] = (S.first && lane * K + k < P.pad) ? P.init : 0.0;
+            }
+            S.gM = S.gI = 0.0;
+            S.gD = (S.first && lane * K - 1 < P.pad) ? P.init : 0.0;
+        }
+        double uM = __shfl_up_sync(kFull, S.M[K - 1], 1);
+        double uI = __shfl_up_sync(kFull, S.I[K - 1], 1);
+        double uD = __shfl_up_sync(kFull, S.D[K - 1], 1);
+        if (lane == 0) {
+            if (S.first) {
+                uM = 0.0;
+                uI = 0.0;
+                uD = P.init;
+            } else {
+                uM = S.nxM;
+                uI = S.nxI;
+                uD = S.nxD;
+                if (c + 1 < P.H) {
+                    S.nxM = above[3 * (c + 1) + 0];
+                    S.nxI = above[3 * (c + 1) + 1];
+                    S.nxD = above[3 * (c + 1) + 2];
+                }
+            }
+        }
+#pragma unroll
+        for (int k = K - 1; k >= 0; --k) {
+            const double dM = k ? S.M[k - 1] : S.gM;
+            const double dI = k ? S.I[k - 1] : S.gI;
+            const double dD = k ? S.D[k - 1] : S.gD;
+            const double prior = (S.base[k] == y || yn) ? S.pm[k] : S.pe[k];
+            double Mn, Dn;
+            if (RESCALED) {
+                Mn = mul64(prior, fma(dI, S.c1[k], fma(dD, S.c2[k], dM)), u);
+                Dn = fma(S.D[k], S.dd[k], S.M[k]);
+            } else {  // the reference's grouping: prior x (M x MM + (I + D) x IM), so results deep in the
+                      // subnormal range round as LoglessPairHMM's do
+                Mn = mul64(prior, fma(dM, S.c1[k], mul64(add64(dI, dD, u), S.c2[k], u)), u);
+                Dn = fma(S.D[k], S.dd[k], mul64(S.M[k], S.c5[k], u));
+            }
+            S.M[k] = Mn;
+            S.D[k] = Dn;
+        }
+        double aM = uM, aI = uI;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double In = RESCALED ? fma(aI, S.c3[k], aM) : fma(aI, S.c4[k], mul64(aM, S.c3[k], u));
+            S.I[k] = In;
+            aM = S.M[k];
+            aI = In;
+        }
+        S.gM = uM;
+        S.gI = uI;
+        S.gD = uD;
+        if (valid && lane == 31) {
+            if (S.last) {
+                rowM[s - s0] = S.M[K - 1];
+                rowI[s - s0] = S.I[K - 1];
+            } else {
+                below[3 * c + 0] = S.M[K - 1];
+                below[3 * c + 1] = S.I[K - 1];
+                below[3 * c + 2] = S.D[K - 1];
+            }
+        }
+    }
+}
+
+// Phase r (steps 16 r .. 16 r + 15) of a strip; the last strip's part of the last row is added to acc, a column per
+// lane.
+template <bool RESCALED>
+__device__ __forceinline__ void strip_phase(const Pair64 &P, Strip64<RESCALED> &S, int r, const double *above,
+                                            double *below, double *rowM, double *rowI, double kappa, double &acc,
+                                            Unit u, int lane) {
+    const int s0 = r * kPhase, s1 = min(s0 + kPhase, P.H + 31);
+    switch (S.k) {
+        case 1: strip_steps<1, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+        case 2: strip_steps<2, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+        case 3: strip_steps<3, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+        default: strip_steps<4, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+    }
+    if (S.last) {
+        __syncwarp();
+        const int c = s0 + lane - 31;
+        if (s0 + lane < s1 && c >= 0 && c < P.H)
+            acc += RESCALED ? fma(kappa, rowI[lane], rowM[lane]) : rowM[lane] + rowI[lane];
+        __syncwarp();
+    }
+}
+
+// The pair's scale (RESCALED): la = log2 a_R and the initial condition divided by 2^round(la); all lanes.
+template <bool RESCALED>
+__device__ __forceinline__ void pair_scale(const DevTables &T, const DevBatch &B, Pair64 &P, double &kappa, int lane) {
+    P.init = B.hap_init_d[P.hap];
+    kappa = 1.0;
+    if (!RESCALED) return;
+    double la = 0.0;
+    for (int p = lane; p < P.R; p += 32) la += __ldg(T.lm2m64 + B.ins[P.roff + p] * 128 + B.dels[P.roff + p]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) la += __shfl_xor_sync(kFull, la, o);
+    P.la = la;
+    P.init = scalbn(P.init, -60 - (int)rint(la));
+    const uint8_t ins = B.ins[P.roff + P.R - 1], del = B.dels[P.roff + P.R - 1];
+    kappa = __ldg(T.err_d + ins) / __ldg(T.m2m_d + ins * 128 + del);
+}
+
+template <bool RESCALED>
+__device__ __forceinline__ void pair_emit(const DevBatch &B, const Pair64 &P, double acc, int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+    if (lane != 0) return;
+    if (RESCALED) {
+        const double rla = rint(P.la);
+        const double v = log10(acc) - kLog10Scale64R - (P.la - rla) * 0.30102999566398120;
+        if (v >= kRescaledFloor && v <= 0.0) {
+            B.out[P.out_index] = v;
+        } else {  // too close to the FP64 range at S' (or not finite): the exact tier recomputes it
+            const int idx = atomicAdd(&B.counters[4], 1);
+            if ((int64_t)idx < B.rerun_capacity)
+                B.rerun[B.rerun_capacity + idx] = PairRef{P.read, P.hap};
+            else
+                atomicExch(&B.counters[3], 1);
+        }
+    } else {
+        B.out[P.out_index] = log10(acc) - kLog10Scale64;
+    }
+}
+
+// A pair that needs no wavefront: an empty read or haplotype (-inf, as in Java), or one beyond the strip scratch.
+__device__ __forceinline__ bool pair_skipped(const DevBatch &B, const Pair64 &P, bool writer) {
+    if (P.R == 0 || P.H == 0) {
+        if (writer) B.out[P.out_index] = -INFINITY;
+        return true;
+    }
+    if (P.H > B.scratch64_cols && P.blocks32 > 1) {
+        if (writer) atomicExch(&B.counters[3], 2);
+        return true;
+    }
+    return false;
+}
+
+// Launched with full grids; queue lengths are device counters, so the choice between a pair per warp and a pair per
+// block is made here.  A pair per block when the list is shorter than the grid's warps (each pair then runs on four
+// sub-partitions) and when the batch has long reads (kFp64SplitRows: a pair's time on one warp, 15 ms at 1,400 x 2,250
+// bases, is what the last pairs of a long list would otherwise take); a pair per warp for long lists of short reads,
+// where the lag of the strips would idle a tenth of the warps.
+template <bool RESCALED>
+__global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables T, DevBatch B, bool long_reads,
+                                                                      Unit u) {
+    __shared__ double row_sum[kWarps64][2][kPhase];
+    __shared__ int job;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const PairRef *queue = RESCALED ? B.rerun : B.rerun + B.rerun_capacity;
+    const int total = min(B.counters[RESCALED ? 1 : 4], (int)B.rerun_capacity);
+    int *const cursor = &B.counters[RESCALED ? 2 : 5];
+    double *const block_scratch = B.scratch64 + (int64_t)blockIdx.x * kWarps64 * B.scratch64_cols * 3;
+    double *const mine = block_scratch + (int64_t)warp * B.scratch64_cols * 3;
+    double *const rowM = row_sum[warp][0], *const rowI = row_sum[warp][1];
+    Strip64<RESCALED> S;
+    double kappa;
+    if (total > (int)gridDim.x * kWarps64 && !long_reads) {
+        for (bool first = true;;) {
+            const int t = draw_entry(cursor, first, lane);
+            if (t >= total) break;
+            Pair64 P = load_pair(B, queue[t]);
+            if (pair_skipped(B, P, lane == 0)) continue;
+            pair_scale<RESCALED>(T, B, P, kappa, lane);
+            const int n = (P.blocks32 + 3) / 4, phases = (P.H + 31 + kPhase - 1) / kPhase;
+            double acc = 0.0;
+            for (int strip = 0; strip < n; ++strip) {
+                __syncwarp();  // the strip above has written its last row
+                strip_begin<RESCALED>(T, B, P, strip, n, mine, S, lane);
+                for (int r = 0; r < phases; ++r) strip_phase<RESCALED>(P, S, r, mine, mine, rowM, rowI, kappa, acc, u, lane);
+            }
+            pair_emit<RESCALED>(B, P, acc, lane);
+        }
+        return;
+    }
+    const double *const above = block_scratch + (int64_t)((warp + kWarps64 - 1) % kWarps64) * B.scratch64_cols * 3;
+    for (bool first = true;;) {
+        int t = blockIdx.x;
+        if (!first) {
+            __syncthreads();  // every warp has read the previous job
+            if (threadIdx.x == 0) job = (int)gridDim.x + atomicAdd(cursor, 1);
+            __syncthreads();
+            t = job;
+        }
+        first = false;
+        if (t >= total) break;
+        Pair64 P = load_pair(B, queue[t]);
+        if (pair_skipped(B, P, threadIdx.x == 0)) continue;
+        pair_scale<RESCALED>(T, B, P, kappa, lane);
+        // strips of at most 128 rows, a multiple of four of them where the rows allow; strip s runs on warp s % 4 from
+        // phase start(s) = (s / 4) round + (s % 4) lag on, round being a strip's phases and long enough for the strip
+        // that wraps round to warp 0 to stay behind the one above it on warp 3
+        const int n = min(((P.blocks32 + 3) / 4 + 3) / 4 * 4, P.blocks32);
+        const int phases = (P.H + 31 + kPhase - 1) / kPhase;
+        const int round = max(phases, kStripLag * kWarps64);
+        const int end = (n - 1) / kWarps64 * round + (n - 1) % kWarps64 * kStripLag + phases;
+        int strip = warp, start = warp * kStripLag;
+        double acc = 0.0;
+        for (int p = 0; p < end; ++p) {
+            if (strip < n && p >= start) {
+                if (p == start) strip_begin<RESCALED>(T, B, P, strip, n, above, S, lane);
+                strip_phase<RESCALED>(P, S, p - start, above, mine, rowM, rowI, kappa, acc, u, lane);
+                if (p - start == phases - 1) {
+                    strip += kWarps64;
+                    start += round;
+                }
+            }
+            __syncthreads();
+        }
+        if (warp == (n - 1) % kWarps64) pair_emit<RESCALED>(B, P, acc, lane);
+    }
+}
+
+}  // namespace
+
+int launch_fp64_queue(const DevTables &t, const DevBatch &b, bool long_reads, int grid, cudaStream_t s) {
+    const Unit u{0.0, 1.0};
+    fp64_queue_kernel<true><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_reads, u);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    fp64_queue_kernel<false><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_reads, u);
+    return (int)cudaGetLastError();
+}
+
+int fp64_kernel_occupancy(int *blocks_per_sm) {
+    // both tiers run on the same grid and scratch: the smaller occupancy of the two
+    int a = 0, b = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fp64_queue_kernel<true>, 32 * kWarps64, 0);
+    if (e != cudaSuccess) return (int)e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fp64_queue_kernel<false>, 32 * kWarps64, 0);
+    *blocks_per_sm = a < b ? a : b;
+    return (int)e;
+}
+
+}  // namespace ghmm

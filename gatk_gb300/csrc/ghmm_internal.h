@@ -13,7 +13,6 @@ namespace ghmm {
 constexpr uint8_t kColFirst = 0x40;
 constexpr uint8_t kColLast = 0x80;
 constexpr int kMaxK32 = 8;      // FP32 kernel: rows per lane (strip = 32*K rows)
-constexpr int kMaxK64 = 4;      // FP64 kernel: rows per lane
 constexpr int kMaxReadLen = 1 << 20;
 constexpr int kNumBucketKeys = 32;       // bucket key = rows per lane (1..8) | 16 for multi-strip
 constexpr int kCounterBucketBase = 8;    // counters[8 + key]: bucket task cursors
@@ -30,6 +29,7 @@ struct DevTables {
     const double *prob_d;
     const double *err3_d;
     const double *m2m_d;
+    const double *lm2m64;   // [128*128] -log2(m2m_d), the rescaled FP64 tier's
     const double *lm2m_d;   // [128*128] -log2(m2m_f), the FP32 pass's row rescaling exponent
 };
 
@@ -81,7 +81,8 @@ struct DevBatch {
 
 // Kernel launchers (kernels.cu).  All return cudaError_t as int.
 int launch_fp32_bucket(const DevTables &t, const DevBatch &b, int key, int grid, int block, cudaStream_t s);
-int launch_fp64_queue(const DevTables &t, const DevBatch &b, int grid, int block, cudaStream_t s);
+int launch_fp64_queue(const DevTables &t, const DevBatch &b, bool long_reads, int grid, cudaStream_t s);  // fp64.cu
+constexpr int kFp64SplitRows = 481;  // batches with reads of this many bases run a pair per block at any queue length
 int launch_finalize_fp32(double *out, const int64_t *n_out, int sm_count, cudaStream_t s);
 // Per-read log2 a_R of the FP32 pass (kernels.cu), into scale[n_reads]; after the read planes are final.
 int launch_read_scale(const DevTables &t, const DevBatch &b, int64_t n_reads, float2 *scale, int sm_count,
@@ -99,7 +100,7 @@ constexpr int kCodePad = 64;
 // this only keeps pairs that would almost surely overflow from running twice).
 constexpr double kMaxGrowth64 = 1e15;
 int fp32_kernel_occupancy(int k, int block, int *blocks_per_sm);
-int fp64_kernel_occupancy(int block, int *blocks_per_sm);
+int fp64_kernel_occupancy(int *blocks_per_sm);
 
 // PD-HMM (pd.cu): per haplotype column, the PD flag byte (PartiallyDeterminedHaplotype bits) and the HMM state
 // code: bits 0-1 the state the read's first row uses at this column, bits 2-3 the state of the other rows

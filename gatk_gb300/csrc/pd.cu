@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "ghmm_internal.h"
+#include "warp_list.cuh"
 
 namespace ghmm {
 namespace {
@@ -82,10 +83,8 @@ __global__ void __launch_bounds__(kPdBlock, (sizeof(V) == 4 && K <= 4) ? 4 : 3) 
     const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     V *scratch = reinterpret_cast<V *>(B.scratch64) + warp_global * B.scratch64_cols * 6;
     if (count_dev) count = min(*count_dev, (int)B.rerun_capacity);
-    for (;;) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(&B.counters[cursor], 1);
-        t = __shfl_sync(kFull, t, 0);
+    for (bool first_entry = true;;) {
+        const int t = draw_entry(&B.counters[cursor], first_entry, lane);
         if (t >= count) break;
         const PairRef pr = B.rerun[begin + t];
         const int read = pr.read, hap = pr.hap;

@@ -155,6 +155,7 @@ int ghmm_initialize(const ghmm_args *args, ghmm_ctx **out) {
     ctx->tables.err3_d = dt->err3;
     ctx->tables.m2m_d = dt->m2m;
     ctx->tables.lm2m_d = dt->lm2m;
+    ctx->tables.lm2m64 = dt->lm2m64;
     ctx->alive = true;
     *out = ctx;
     return GHMM_OK;

@@ -73,6 +73,7 @@ void build_host_tables(HostTables &t) {
     }
     for (int k = 0; k < 128 * 128; k++) {
         t.m2m_f[k] = (float)t.m2m[k];
+        t.lm2m64[k] = t.m2m[k] > 0.0 ? -std::log2(t.m2m[k]) : 0.0;  // MM = 0 reads run in the exact tier only
         t.lm2m[k] = t.m2m_f[k] > 0.0f ? -std::log2((double)t.m2m_f[k]) : 0.0;  // MM = 0 reads never run in FP32
     }
 }

@@ -1,0 +1,71 @@
+"""How a call's work is split must not show in its results: FP64 pairs on one warp or one block, strips of any height,
+and regions cut into more or fewer FP32 tasks."""
+import numpy as np
+import pytest
+
+from gatk_gb300 import native, workload
+from gatk_gb300.pairhmm import Engine
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _reads(rng, lengths, ins=(30, 46)):
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    return [(acgt[rng.integers(0, 4, n)], rng.integers(6, 41, n), rng.integers(*ins, n), rng.integers(*ins, n),
+             np.full(n, 10)) for n in lengths]
+
+
+def _region(rng, read_lengths, hap_lengths, ins=(30, 46)):
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    return [acgt[rng.integers(0, 4, n)] for n in hap_lengths], _reads(rng, read_lengths, ins)
+
+
+EDGES = [1, 2, 31, 32, 33, 64, 65, 96, 97, 128, 129, 160, 161, 192, 224, 255, 256, 257, 289, 384, 385]
+
+
+@pytest.mark.parametrize("case", ["pair_per_block", "pair_per_warp", "long_reads", "exact_tier"])
+def test_fp64_strip_shapes(case):
+    """Reads at the edges of the strips' heights, haplotypes at the edges of the 16-column phases.  |d| <= 1e-9 is the
+    repository's bar for FP64 results."""
+    rng = np.random.default_rng(11)
+    haps = [1, 2, 15, 16, 17, 31, 32, 33, 48, 97]
+    if case == "pair_per_block":
+        regions = [_region(rng, EDGES, haps)]
+    elif case == "pair_per_warp":  # more pairs than any grid has warps, no read of 481 bases or more
+        regions = [_region(rng, EDGES, haps) for _ in range(16)]
+    elif case == "long_reads":
+        regions = [_region(rng, [480, 481, 512, 513, 640, 1025, 1537, 2049], [1, 16, 130, 700])]
+    else:  # insertion and deletion penalties of Phred 3: matchToMatch about 0, every pair in the unscaled tier
+        regions = [_region(rng, EDGES, haps, ins=(3, 4))]
+    wl = workload.from_pairs(regions)
+    eng = Engine(use_double_precision=True)
+    try:
+        got = eng.compute(wl)
+    finally:
+        eng.close()
+    want = oracle.compute_workload(wl)
+    same = got == want  # equal infinities
+    assert np.max(np.abs(np.where(same, 0.0, got - want))) <= 1e-9
+
+
+def test_results_do_not_depend_on_the_task_split():
+    """Regions called one by one (cut down to a haplotype a task) and in one batch of many (whole regions a task) give
+    the same bits, several strips included."""
+    rng = np.random.default_rng(12)
+    few = [_region(rng, [40, 150, 151, 254, 255, 300, 520], [700, 640, 655, 610, 620]),
+           _region(rng, [1, 30, 31, 62, 63], [90]), _region(rng, [100, 101, 102], [333] * 9)]
+    eng = Engine()
+    try:
+        alone = [eng.compute(workload.from_pairs([r])) for r in few]
+        big = workload.generate(1, regions=400)
+        haps_reads = [([big.hap(h) for h in range(int(big.region_hap_off[g]), int(big.region_hap_off[g + 1]))],
+                       [big.read(r) for r in range(int(big.region_read_off[g]), int(big.region_read_off[g + 1]))])
+                      for g in range(0, 400, 4)]
+        wl = workload.from_pairs(few + haps_reads * 4)
+        with eng.batch(wl) as b:
+            b.forward(native.MODE_FP32_RERUN)
+            together = b.results()
+    finally:
+        eng.close()
+    assert np.array_equal(np.concatenate(alone), together[:sum(len(a) for a in alone)])
