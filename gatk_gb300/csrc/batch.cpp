@@ -170,25 +170,37 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
     std::vector<int64_t> region_strips((size_t)G, 0);  // strips of the region's reads (FP32 layout)
     const HostTables &HT = *ctx->host_tables;
 
-    parallel_for(G, threads, [&](int64_t g) {
-        int64_t r = rro[(size_t)g];
+    // a region's reads in blocks of up to 64, so that one deep region spreads over the cores too
+    struct ReadBlock {
+        int64_t g, r0, r1;
+        int max_read;
+        int64_t strips;  // of its reads (FP32 layout)
+    };
+    std::vector<ReadBlock> blocks;
+    blocks.reserve((size_t)(G + NR / 64));
+    for (int64_t g = 0; g < G; g++)
+        for (int64_t r = rro[(size_t)g]; r < rro[(size_t)g + 1]; r += 64)
+            blocks.push_back(ReadBlock{g, r, std::min(r + 64, rro[(size_t)g + 1]), 0, 0});
+    parallel_for((int64_t)blocks.size(), threads, [&](int64_t i) {
+        ReadBlock &block = blocks[(size_t)i];
+        const int64_t g = block.g;
         int mx = 0;
         int64_t hmin = INT64_MAX;
         for (int64_t h = rho[(size_t)g]; h < rho[(size_t)g + 1]; h++)
             hmin = std::min<int64_t>(hmin, hap_off[(size_t)h + 1] - hap_off[(size_t)h]);
         const double max_i_scaled = 1e37 * (double)std::max<int64_t>(hmin, 1) / std::ldexp(1.0, 120);
-        for (int64_t k = 0; r < rro[(size_t)g + 1]; r++, k++) {
+        for (int64_t r = block.r0; r < block.r1; r++) {
             const int64_t ofs = read_off[(size_t)r];
             const int R = (int)(read_off[(size_t)r + 1] - ofs);
             mx = std::max(mx, R);
-            region_strips[(size_t)g] += (R + kAccRows + 32 * kMaxK32 - 1) / (32 * kMaxK32);
+            block.strips += (R + kAccRows + 32 * kMaxK32 - 1) / (32 * kMaxK32);
             const uint8_t *sb, *sq, *si, *sd, *sg;
             if (src.flat) {
                 const ghmm_flat *f = src.flat;
                 const int64_t so = f->read_off[f->region_read_off[0] + r];
                 sb = f->bases + so; sq = f->quals + so; si = f->ins_gop + so; sd = f->del_gop + so; sg = f->gcp + so;
             } else {
-                const ghmm_read &rd = src.regions[g].reads[k];
+                const ghmm_read &rd = src.regions[g].reads[r - rro[(size_t)g]];
                 sb = rd.bases; sq = rd.quals; si = rd.ins_gop; sd = rd.del_gop; sg = rd.gcp;
             }
             if (R > 0) {
@@ -223,7 +235,13 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
             read_flag[(size_t)r] = fl;
             b.h_read_region.p[r] = (int32_t)g;
         }
-        region_max_read[(size_t)g] = mx;
+        block.max_read = mx;
+    });
+    for (const ReadBlock &block : blocks) {
+        region_max_read[(size_t)block.g] = std::max(region_max_read[(size_t)block.g], block.max_read);
+        region_strips[(size_t)block.g] += block.strips;
+    }
+    parallel_for(G, threads, [&](int64_t g) {
         for (int64_t h = rho[(size_t)g]; h < rho[(size_t)g + 1]; h++) {
             const int64_t ofs = hap_off[(size_t)h];
             const int H = (int)(hap_off[(size_t)h + 1] - ofs);
@@ -413,7 +431,7 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
     }
     total_tasks = bucket_pos[kNumBucketKeys];
     GHMM_CUDA(b.h_tasks.reserve((size_t)std::max<int64_t>(total_tasks, 1)), "pinned tasks");
-    parallel_for(kNumBucketKeys, threads, [&](int64_t key) {
+    parallel_for(kNumBucketKeys, total_tasks < 2048 ? 1 : threads, [&](int64_t key) {
         const int64_t n = bucket_pos[(size_t)key + 1] - bucket_pos[(size_t)key];
         if (n == 0) return;
         std::vector<std::pair<int64_t, int64_t>> order;  // (-cost, position in region order)

@@ -15,6 +15,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "ghmm_internal.h"
+#include "host_pool.h"
 
 struct ghmm_ctx;
 struct ghmm_batch;
@@ -33,6 +34,9 @@ struct NvtxRange {
 // Test hook (ghmm_debug_inject): the number of device allocations still to be refused as out of memory
 extern std::atomic<int64_t> g_refuse_allocations;
 
+// Frees the buffers that contexts keep of destroyed batches (runtime.cpp); false when there were none.
+bool release_spare_batches();
+
 template <typename T>
 struct DevBuf {
     T *p = nullptr;
@@ -48,6 +52,10 @@ struct DevBuf {
         p = nullptr;
         cap = 0;
         cudaError_t e = cudaMalloc(&p, want * sizeof(T));
+        if (e == cudaErrorMemoryAllocation && release_spare_batches()) {
+            cudaGetLastError();  // the failed attempt's
+            e = cudaMalloc(&p, want * sizeof(T));
+        }
         if (e == cudaSuccess) cap = want;
         return e;
     }
@@ -69,6 +77,10 @@ struct HostBuf {  // pinned
         p = nullptr;
         cap = 0;
         cudaError_t e = cudaMallocHost(&p, want * sizeof(T));
+        if (e == cudaErrorMemoryAllocation && release_spare_batches()) {
+            cudaGetLastError();
+            e = cudaMallocHost(&p, want * sizeof(T));
+        }
         if (e == cudaSuccess) cap = want;
         return e;
     }
@@ -86,7 +98,8 @@ inline int hw_threads(int requested) {
 
 // f(i) for i in [0, n) on up to `threads` threads, the calling thread one of them.  Threads take `grain`
 // consecutive indices at a time; grain 0 (the default) takes about a quarter of an even share, at most 64, so
-// that a loop over a few dozen regions or blocks still spreads over all threads.
+// that a loop over a few dozen regions or blocks still spreads over all threads.  The other threads are the pool's
+// (host_pool.h), or started for this loop where there is no pool.
 template <typename F>
 inline void parallel_for(int64_t n, int threads, F f, int64_t grain = 0) {
     if (n <= 0) return;
@@ -106,6 +119,10 @@ inline void parallel_for(int64_t n, int threads, F f, int64_t grain = 0) {
             for (int64_t i = i0; i < i1; i++) f(i);
         }
     };
+    if (const auto hosts = HostPool::get()) {
+        hosts->run(threads - 1, work);
+        return;
+    }
     std::vector<std::thread> pool;
     pool.reserve((size_t)threads - 1);
     for (int t = 1; t < threads; t++) pool.emplace_back(work);

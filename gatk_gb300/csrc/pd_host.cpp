@@ -281,6 +281,7 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s) 
             const unsigned char *k3 = (const unsigned char *)kg;
             sig.insert(sig.end(), k3, k3 + sizeof(kg));
         }
+        sig.push_back(1);  // (of odd length, unlike the regular forward's)
         if (sig != b.graph_sig) {
             if (b.graph[0]) cudaGraphExecDestroy(b.graph[0]);
             b.graph[0] = nullptr;
@@ -433,7 +434,7 @@ int ghmm_pd_batch_create(ghmm_ctx *ctx, const ghmm_pd_region *regions, int32_t n
     if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
     if (!out || n_regions < 0 || (n_regions > 0 && !regions)) return fail(ctx, GHMM_ERR_ARG, "bad arguments");
     GHMM_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
-    auto *b = new ghmm_batch();
+    auto *b = new_batch(ctx);
     int rc = pd_marshal(ctx, regions, n_regions, *b, nullptr);
     if (!rc) rc = pd_upload(ctx, *b, ctx->stream);
     if (!rc) rc = cudaStreamSynchronize(ctx->stream) == cudaSuccess ? GHMM_OK : fail(ctx, GHMM_ERR_CUDA, "upload");
@@ -475,7 +476,7 @@ int ghmm_pd_batch_create_raw(ghmm_ctx *ctx, const ghmm_pd_raw_region *regions, i
     if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
     if (!out || n_regions < 0 || (n_regions > 0 && !regions)) return fail(ctx, GHMM_ERR_ARG, "bad arguments");
     GHMM_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
-    auto *b = new ghmm_batch();
+    auto *b = new_batch(ctx);
     int rc = pd_raw_build(ctx, regions, n_regions, prep, *b);
     if (!rc) rc = cudaStreamSynchronize(ctx->stream) == cudaSuccess ? GHMM_OK : fail(ctx, GHMM_ERR_CUDA, "upload");
     if (rc) {

@@ -200,7 +200,7 @@ int ghmm_batch_create_raw(ghmm_ctx *ctx, const ghmm_raw_region *regions, int32_t
     RawView v;
     int rc = raw_view(ctx, regions, n_regions, prep, v);
     if (rc) return rc;
-    auto *b = new ghmm_batch();
+    auto *b = new_batch(ctx);
     Source src;
     src.regions = v.regions.data();
     src.n_regions = n_regions;

@@ -55,7 +55,67 @@ int cuda_fail(ghmm_ctx *ctx, cudaError_t e, const char *what) {
 }
 
 
+// The buffers of each open context's last destroyed batch, for its next one: a program that makes a batch per group of
+// regions otherwise allocates and frees some thirty pinned and device buffers each time (150 regions: 5 of the 18 ms
+// from raw reads to cigars).  At most one batch a context, of at most kSpareBytes; given back when the context closes,
+// and by any allocation of the process that fails (release_spare_batches).
+struct SpareBatch {
+    uint64_t ctx_id;
+    int device;
+    ghmm_batch *b;
+};
+constexpr size_t kSpareBytes = (size_t)1 << 30;
+std::mutex g_spare_mu;
+std::vector<SpareBatch> g_spares;
+
+ghmm_batch *take_spare(uint64_t ctx_id) {
+    std::lock_guard<std::mutex> lk(g_spare_mu);
+    for (size_t i = 0; i < g_spares.size(); i++)
+        if (g_spares[i].ctx_id == ctx_id) {
+            ghmm_batch *b = g_spares[i].b;
+            g_spares.erase(g_spares.begin() + (ptrdiff_t)i);
+            return b;
+        }
+    return nullptr;
+}
+
+ghmm_batch *new_batch(ghmm_ctx *ctx) {
+    ghmm_batch *b = take_spare(ctx->id);
+    if (!b) b = new ghmm_batch();
+    b->ctx_id = ctx->id;
+    return b;
+}
+
+// Keeps b, whose work on the device is done, for the context's next batch; false: not kept.
+bool keep_spare(ghmm_ctx *ctx, ghmm_batch *b) {
+    if (b->buffer_bytes() > kSpareBytes) return false;
+    b->recycle();
+    if (ghmm_batch *old = take_spare(ctx->id)) {
+        old->release();
+        delete old;
+    }
+    std::lock_guard<std::mutex> lk(g_spare_mu);
+    g_spares.push_back(SpareBatch{ctx->id, ctx->device, b});
+    return true;
+}
+
 }  // namespace rt
+
+bool release_spare_batches() {
+    std::lock_guard<std::mutex> lk(rt::g_spare_mu);
+    if (rt::g_spares.empty()) return false;
+    int device = 0;
+    cudaGetDevice(&device);
+    for (auto &s : rt::g_spares) {
+        cudaSetDevice(s.device);
+        s.b->release();
+        delete s.b;
+    }
+    rt::g_spares.clear();
+    cudaSetDevice(device);
+    return true;
+}
+
 }  // namespace ghmm
 
 void ghmm::set_global_error(const char *msg) {
@@ -156,6 +216,9 @@ int ghmm_initialize(const ghmm_args *args, ghmm_ctx **out) {
     ctx->tables.m2m_d = dt->m2m;
     ctx->tables.lm2m_d = dt->lm2m;
     ctx->tables.lm2m64 = dt->lm2m64;
+    static std::atomic<uint64_t> next_id{1};
+    ctx->id = next_id.fetch_add(1);
+    HostPool::retain();
     ctx->alive = true;
     *out = ctx;
     return GHMM_OK;
@@ -253,6 +316,10 @@ int ghmm_done(ghmm_ctx *ctx) {
     if (ctx->pipe) queue_close(ctx->pipe);
     ctx->pipe = nullptr;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ghmm_batch *spare = take_spare(ctx->id)) {
+        spare->release();
+        delete spare;
+    }
     ctx->scratch_batch.release();
     for (auto &pb : ctx->pd_batch) pb.release();
     ctx->calib_scratch.release();
@@ -271,6 +338,7 @@ int ghmm_done(ghmm_ctx *ctx) {
     for (auto &ev : ctx->fork_ev)
         if (ev) cudaEventDestroy(ev);
     delete ctx;
+    HostPool::release();
     return GHMM_OK;
 }
 
@@ -309,7 +377,7 @@ int ghmm_compute_likelihoods(ghmm_ctx *ctx, const ghmm_read *reads, int32_t n_re
 int ghmm_batch_create(ghmm_ctx *ctx, const ghmm_region *regions, int32_t n_regions, ghmm_batch **out) {
     if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
     if (!out || n_regions < 0 || (n_regions > 0 && !regions)) return fail(ctx, GHMM_ERR_ARG, "bad arguments");
-    auto *b = new ghmm_batch();
+    auto *b = new_batch(ctx);
     Source src;
     src.regions = regions;
     src.n_regions = n_regions;
@@ -328,7 +396,7 @@ int ghmm_batch_create(ghmm_ctx *ctx, const ghmm_region *regions, int32_t n_regio
 int ghmm_batch_create_flat(ghmm_ctx *ctx, const ghmm_flat *flat, ghmm_batch **out) {
     if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
     if (!out || !flat || flat->n_regions < 0) return fail(ctx, GHMM_ERR_ARG, "bad arguments");
-    auto *b = new ghmm_batch();
+    auto *b = new_batch(ctx);
     Source src;
     src.flat = flat;
     src.n_regions = flat->n_regions;
@@ -430,8 +498,10 @@ int ghmm_batch_destroy(ghmm_ctx *ctx, ghmm_batch *b) {
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
     }
-    b->release();
-    delete b;
+    if (!ctx || !ctx->alive || b->ctx_id != ctx->id || !keep_spare(ctx, b)) {
+        b->release();
+        delete b;
+    }
     return GHMM_OK;
 }
 

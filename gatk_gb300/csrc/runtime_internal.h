@@ -127,6 +127,7 @@ struct ghmm_batch {
     double ms_fp32 = 0, ms_fp64 = 0, ms_plain = 0, ms_total = 0;
     int64_t upload_bytes = 0, forward_h2d = 0, forward_d2h = 0, results_d2h = 0;
     bool uploaded = false;
+    uint64_t ctx_id = 0;  // the context that created it (batch handles)
     DevBatch dev{};
     // asynchronous forward: events of the last enqueue, and the captured launch sequence
     cudaEvent_t ev[5]{};
@@ -137,6 +138,29 @@ struct ghmm_batch {
     int pending_mode = -1;
     cudaGraphExec_t graph[2]{};  // captured FP32 phase (PD batches: its packed buckets) and FP64 phase
     std::vector<unsigned char> graph_sig;  // DevBatch bytes, mode, bucket keys and grids the graphs were captured for
+
+    // bytes of the pinned and device buffers
+    size_t buffer_bytes() const {
+        size_t n = 0;
+        auto add = [&n](const auto &...buf) { ((n += buf.cap * sizeof(*buf.p)), ...); };
+        add(h_planes, h_hap, h_off, h_read_region, h_init_f, h_init_d, h_tasks, h_direct, h_fp64all, h_out, h_counters,
+            h_nout, d_planes, d_hap, d_off, d_read_region, d_init_f, d_init_d, d_tasks, d_rerun, d_out, d_counters, d_nout,
+            d_post, h_mapq, d_mapq, h_dragstr, d_dragstr, h_pd, d_pd, d_scratch32, d_scratch64, d_read_scale);
+        return n;
+    }
+
+    // As a new batch, but for the buffers, events and captured graphs it keeps
+    void recycle() {
+        has_pd = uploaded = prep_timed = false;
+        n_regions = n_reads = n_haps = read_bytes = hap_bytes = n_out = n_cells = 0;
+        n_tasks = n_direct = n_direct_exact = cells_direct = 0;
+        buckets.clear();
+        last_mode = pending_mode = -1;
+        last_launches = 0;
+        last_rerun = last_exact = pending_n_pre = 0;
+        ms_fp32 = ms_fp64 = ms_plain = ms_total = ms_host_copy = ms_host_tasks = 0;
+        upload_bytes = forward_h2d = forward_d2h = results_d2h = 0;
+    }
 
     void release() {
         for (auto &g : graph) {
@@ -164,6 +188,7 @@ struct ghmm_batch {
 };
 
 struct ghmm_ctx {
+    uint64_t id = 0;  // unique in the process: the owner of spare batches
     int64_t debug_force_rerun = 0;  // test hook: every n-th FP32 output rerun in FP64 (batches uploaded afterwards)
     int device = 0;
     int sm_count = 0;
@@ -294,6 +319,8 @@ struct RawView {
 };
 
 // runtime.cpp: status and message of a failed call (into the queue worker's own message on its thread)
+// runtime.cpp: a batch for a new handle, with the buffers of the context's last destroyed one where it kept them
+ghmm_batch *new_batch(ghmm_ctx *ctx);
 extern thread_local std::string *t_error_sink;
 int fail(ghmm_ctx *ctx, int code, const std::string &msg);
 int cuda_fail(ghmm_ctx *ctx, cudaError_t e, const char *what);
