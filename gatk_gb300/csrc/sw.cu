@@ -16,7 +16,7 @@
 //                         vertical gap opened here; horizontal gap opened here), from which the traceback rebuilds
 //                         the backtrack entry 0 / -ki / +kd exactly: a gap's length is the distance to the cell that
 //                         opened it.  The last column's and the bottom row's scores go to an edge array.
-//   sw_traceback_kernel   one thread per alignment: end cell per strategy, traceback, cigar elements in reverse
+//   sw_traceback_kernel   one warp per alignment: end cell per strategy, traceback, cigar elements in reverse
 //                         into a per-pair slot (calculateCigar, :261-379).
 //   sw_scan_*_kernel      exclusive prefix sums of per-pair element counts and the copy into one compact array of
 //                         forward-ordered BAM-encoded cigar ops.
@@ -434,52 +434,53 @@ __global__ void __launch_bounds__(128) sw_prepass_kernel(SwArgs A, int n_pairs) 
     }
 }
 
-// traceback bits of cell (i, j), 1-based
-// Traceback bits of cell (i, j), 1-based.  Keeps the last 16-byte group (4 steps of one lane) it loaded: walks move
-// one step back per cell along a lane, so most cells come from the group already held.
+// Traceback bits of cell (i, j), 1-based.
 struct TbReader {
     const uint32_t *base;  // the alignment's words
     int64_t strip_words;
     int K;
-    int64_t held = -1;     // word index of the group held
-    uint4 g;
-    __device__ __forceinline__ uint32_t code(int i, int j) {
+    __device__ __forceinline__ uint32_t code(int i, int j) const {
         const int w = 32 * K;
         const int s = (j - 1) / w, within = (j - 1) - s * w;
         const int lane = within / K, k = within - lane * K;
         const int64_t t = (int64_t)(i - 1) + lane;
-        const int64_t grp = (int64_t)s * strip_words + ((t >> 2) * 32 + lane) * 4;
-        if (grp != held) {
-            g = *reinterpret_cast<const uint4 *>(base + grp);
-            held = grp;
-        }
-        const int q = (int)(t & 3);
-        const uint32_t word = q == 0 ? g.x : q == 1 ? g.y : q == 2 ? g.z : g.w;
+        const uint32_t word = __ldg(base + (int64_t)s * strip_words + ((t >> 2) * 32 + lane) * 4 + (t & 3));
         return (word >> (4 * k)) & 15u;
     }
 };
 
-__global__ void sw_traceback_kernel(SwArgs A, int n_pairs) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// End cell, traceback and cigar of one alignment by one warp.  Both walks are chains of dependent loads from memory
+// (half a microsecond each), so the lanes look ahead together: the end cell's scores 32 at a time, the next 32 cells
+// down the diagonal (a path is diagonal but for its few gaps), the next 32 cells along a gap.  One thread per
+// alignment took 0.63 ms however few the alignments (reads of 100-250 bases against haplotypes of 200-600); the device
+// time of 54,000 of them in two passes fell from 4.38 to 3.43 ms with a warp each.
+__global__ void __launch_bounds__(128) sw_traceback_kernel(SwArgs A, int n_pairs) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int p = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     if (p >= n_pairs) return;
+    const int lane = threadIdx.x & 31;
     const SwPair P = A.pairs[p];
     const int n = P.ref_len, m = P.alt_len;
     uint32_t *slot = A.slot + P.slot_off;
     const int cap = 2 * m + 4;
-    if (n <= 0) {           // a read whose region has no haplotype: not aligned
-        A.n_ops[p] = 0;
-        A.offset[p] = -1;
+    const int st = n > 0 ? A.state[p] : 0;  // 1: shortcut; 0: int32 scores; 2 / 3: 16-bit pairs, low / high half
+    if (n <= 0) {                           // a read whose region has no haplotype: not aligned
+        if (lane == 0) {
+            A.n_ops[p] = 0;
+            A.offset[p] = -1;
+        }
         return;
     }
-    if (A.state[p] == 1) {  // exact-substring shortcut: cigar mM, offset already written
-        slot[0] = ((uint32_t)m << 4) | kSwOpM;
-        A.n_ops[p] = 1;
+    if (st == 1) {  // exact-substring shortcut: cigar mM, offset already written
+        if (lane == 0) {
+            slot[0] = ((uint32_t)m << 4) | kSwOpM;
+            A.n_ops[p] = 1;
+        }
         return;
     }
     const int K = P.k;
     const int stride = kSwRowStride(K);
     const int km = (m - 1) % (32 * K) % K;  // the last column's place among its lane's columns
-    const int st = A.state[p];              // 0: int32 scores; 2 / 3: 16-bit pairs, low / high half
     const int *lastcol = A.edges + P.edge_off + km, *bottom = A.edges + P.edge_off + (int64_t)n * stride;
     // a stored score (H + open, or its biased 16-bit half) back to H
     auto score = [&](int w) -> int {
@@ -487,41 +488,67 @@ __global__ void sw_traceback_kernel(SwArgs A, int n_pairs) {
         else if (st == 3) w = hi16((uint32_t)w);
         return wsub(w, A.open);
     };
-    int p1 = 0, p2 = 0;
-    int maxscore = INT32_MIN;
+    int p1 = n, p2 = m;
     int segment = 0;
-    if (A.strategy == kSwIndel) {
-        p1 = n;
-        p2 = m;
-    } else {
-        p2 = m;
-        for (int i = 1; i <= n; ++i) {
+    if (A.strategy != kSwIndel) {
+        // last column: the highest score, the lowest row on ties
+        int best = INT32_MIN, row = 0;
+        for (int i = lane + 1; i <= n; i += 32) {
             const int sc = score(lastcol[(int64_t)(i - 1) * stride]);
-            if (sc >= maxscore) {
-                p1 = i;
-                maxscore = sc;
+            if (sc >= best) {
+                best = sc;
+                row = i;
             }
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int b2 = __shfl_xor_sync(kAll, best, o), r2 = __shfl_xor_sync(kAll, row, o);
+            if (b2 > best || (b2 == best && r2 > row)) {
+                best = b2;
+                row = r2;
+            }
+        }
+        p1 = row;
         if (A.strategy != kSwLeadingIndel) {
-            for (int j = 1; j <= m; ++j) {
+            // bottom row: the highest score, on ties the column nearest the main diagonal's, then the first; it
+            // replaces the last column's cell when it scores more, or as much from nearer the diagonal
+            auto off_diagonal = [&](int j) { return n - j < 0 ? j - n : n - j; };
+            int top = INT32_MIN, col = 0, dist = INT32_MAX;
+            for (int j = lane + 1; j <= m; j += 32) {
                 const int sc = score(bottom[(int64_t)((j - 1) / K) * stride + (j - 1) % K]);
-                const int dn = n - j < 0 ? j - n : n - j, dc = p1 - p2 < 0 ? p2 - p1 : p1 - p2;
-                if (sc > maxscore || (sc == maxscore && dn < dc)) {
-                    p1 = n;
-                    p2 = j;
-                    maxscore = sc;
-                    segment = m - j;
+                const int d = off_diagonal(j);
+                if (col == 0 || sc > top || (sc == top && d < dist)) {
+                    top = sc;
+                    col = j;
+                    dist = d;
                 }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int t2 = __shfl_xor_sync(kAll, top, o), c2 = __shfl_xor_sync(kAll, col, o);
+                const int d2 = __shfl_xor_sync(kAll, dist, o);
+                if (c2 > 0 && (col == 0 || t2 > top || (t2 == top && (d2 < dist || (d2 == dist && c2 < col))))) {
+                    top = t2;
+                    col = c2;
+                    dist = d2;
+                }
+            }
+            const int dc = p1 - p2 < 0 ? p2 - p1 : p1 - p2;
+            if (col > 0 && (top > best || (top == best && dist < dc))) {
+                p1 = n;
+                p2 = col;
+                segment = m - col;
             }
         }
     }
     int count = 0;
     bool overflow = false;
-    auto push = [&](int op, int len) {
-        if (count < cap)
-            slot[count] = ((uint32_t)len << 4) | (uint32_t)op;
-        else
+    auto push = [&](int op, int len) {  // (all lanes count, one writes)
+        if (count < cap) {
+            if (lane == 0) slot[count] = ((uint32_t)len << 4) | (uint32_t)op;
+        } else {
             overflow = true;
+        }
         ++count;
     };
     if (segment > 0 && A.strategy == kSwSoftclip) {
@@ -533,39 +560,45 @@ __global__ void sw_traceback_kernel(SwArgs A, int n_pairs) {
     rd.strip_words = sw_steps4(n) * 32;
     rd.K = K;
     int state = kSwOpM;
-    int guard = n + m + 2;
-    do {
-        const uint32_t c = rd.code(p1, p2);
-        int ns, step = 1;
-        if (!(c & 1u)) {
-            ns = kSwOpM;
-        } else if (c & 2u) {  // horizontal: the gap's length is the distance back to the cell that opened it
-            ns = kSwOpI;
-            int q = p2;
-            while (q > 1 && !(rd.code(p1, q) & 8u)) --q;
-            step = p2 - q + 1;
-        } else {              // vertical
-            ns = kSwOpD;
-            int r = p1;
-            while (r > 1 && !(rd.code(r, p2) & 4u)) --r;
-            step = p1 - r + 1;
+    auto take = [&](int op, int len) {
+        if (op == state) {
+            segment += len;
+            return;
         }
-        if (ns == kSwOpM) {
-            --p1;
-            --p2;
-        } else if (ns == kSwOpI) {
-            p2 -= step;
-        } else {
-            p1 -= step;
+        if (segment > 0) push(state, segment);
+        segment = len;
+        state = op;
+    };
+    while (p1 > 0 && p2 > 0) {  // every round moves at least one cell back
+        const bool inside = p1 > lane && p2 > lane;
+        const uint32_t c = inside ? rd.code(p1 - lane, p2 - lane) : 0u;
+        const unsigned stop = __ballot_sync(kAll, !inside || (c & 1u));
+        const int run = stop ? __ffs(stop) - 1 : 32;
+        if (run > 0) take(kSwOpM, run);
+        p1 -= run;
+        p2 -= run;
+        if (run == 32 || p1 <= 0 || p2 <= 0) continue;
+        const bool horizontal = (__shfl_sync(kAll, c, run) & 2u) != 0;
+        const uint32_t opened = horizontal ? 8u : 4u;
+        const int last = horizontal ? p2 : p1;  // the gap's length is the distance back to the cell that opened it
+        int len = 0;
+        for (;;) {
+            const int q = last - len - lane;
+            bool open_here = q <= 1;
+            if (q > 1) open_here = (rd.code(horizontal ? p1 : q, horizontal ? q : p2) & opened) != 0;
+            const unsigned b = __ballot_sync(kAll, open_here);
+            if (b) {
+                len += __ffs(b);
+                break;
+            }
+            len += 32;
         }
-        if (ns == state) {
-            segment += step;
-        } else {
-            if (segment > 0) push(state, segment);
-            segment = step;
-            state = ns;
-        }
-    } while (p1 > 0 && p2 > 0 && --guard > 0);
+        take(horizontal ? kSwOpI : kSwOpD, len);
+        if (horizontal)
+            p2 -= len;
+        else
+            p1 -= len;
+    }
     int off;
     if (A.strategy == kSwSoftclip) {
         push(state, segment);
@@ -582,7 +615,8 @@ __global__ void sw_traceback_kernel(SwArgs A, int n_pairs) {
             push(kSwOpI, p2);
         off = 0;
     }
-    if (overflow || guard <= 0) {
+    if (lane != 0) return;
+    if (overflow) {
         atomicExch(A.error, 1);
         count = 0;
     }
@@ -867,7 +901,7 @@ int sw_forward_occupancy(int k, int *blocks_per_sm) {
 
 int launch_sw_traceback(const SwArgs &a, int n_pairs, cudaStream_t s) {
     if (n_pairs <= 0) return 0;
-    sw_traceback_kernel<<<(n_pairs + 127) / 128, 128, 0, s>>>(a, n_pairs);
+    sw_traceback_kernel<<<(n_pairs + 3) / 4, 128, 0, s>>>(a, n_pairs);
     return (int)cudaGetLastError();
 }
 
