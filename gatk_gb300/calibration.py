@@ -71,6 +71,7 @@ class CalibrationSet:
             a, b = int(wl.read_off[r]), int(wl.read_off[r + 1])
             idx[a:b] = str_parameter_index(wl.bases[a:b])
         self.param_index_np = idx
+        self.max_index = int(idx.max()) if len(idx) else -1
         t = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a).astype(dt)).to(self.device)
         self.bases = t(wl.bases, np.uint8)
         self.quals = t(wl.quals, np.uint8)
@@ -90,6 +91,7 @@ class CalibrationSet:
         """(gap_open, gap_cont) per read position from the [8, 20, 2] table (differentiable in theta)."""
         import torch
 
+        # (log10_likelihoods gathers through ghmm_calib_gather instead; this form is torch operations throughout.)
         # gathered in FP64 so that the backward's index_add sums the 10^5-10^6 per-position gradients into the
         # table in FP64 (index_select's backward is an atomic index_add; advanced indexing's sorts the
         # positions and costs tens of milliseconds)
@@ -145,15 +147,60 @@ def _function():
     return PairHMMLog10Likelihood
 
 
+def _penalties_function():
+    import torch
+
+    class PositionPenalties(torch.autograd.Function):
+        """position_params from the flat FP64 table, by the library's kernels on torch's stream: the values are those of
+        the torch operations, the gradient sums the positions of a table row in FP64 (ghmm_calib_fold)."""
+
+        @staticmethod
+        def forward(ctx, flat, cs, engine):
+            index = cs.param_index.contiguous()
+            n = index.numel()
+            if flat.shape[0] <= cs.max_index:
+                raise IndexError(f"a table of {flat.shape[0]} rows for indices up to {cs.max_index}")
+            table = flat.detach().contiguous()
+            g = torch.empty(n, dtype=torch.float32, device=cs.device)
+            c = torch.empty(n, dtype=torch.float32, device=cs.device)
+            native.check(engine.L.ghmm_calib_gather(engine.handle, table.data_ptr(), table.shape[0], index.data_ptr(), n,
+                                                    LAST_GAP_OPEN, LAST_GAP_CONT, g.data_ptr(), c.data_ptr(),
+                                                    torch.cuda.current_stream(cs.device).cuda_stream), engine.handle)
+            ctx.cs, ctx.engine, ctx.rows = cs, engine, table.shape[0]
+            return g, c
+
+        @staticmethod
+        def backward(ctx, grad_g, grad_c):
+            cs, engine = ctx.cs, ctx.engine
+            index = cs.param_index.contiguous()
+            grad_g, grad_c = (x.detach().to(torch.float32).contiguous() for x in (grad_g, grad_c))
+            out = torch.empty(ctx.rows, 2, dtype=torch.float64, device=cs.device)
+            native.check(engine.L.ghmm_calib_fold(engine.handle, index.data_ptr(), index.numel(), grad_g.data_ptr(),
+                                                  grad_c.data_ptr(), ctx.rows, out.data_ptr(),
+                                                  torch.cuda.current_stream(cs.device).cuda_stream), engine.handle)
+            return out, None, None
+
+    return PositionPenalties
+
+
 _FN = None
+_PENALTIES = None
 
 
 def log10_likelihoods(theta, cs: CalibrationSet, engine, precision: int = 0):
     """Per-pair log10 likelihood under the table theta (differentiable)."""
-    global _FN
+    import torch
+
+    global _FN, _PENALTIES
     if _FN is None:
         _FN = _function()
-    g, c = cs.position_params(theta)
+    if _PENALTIES is None:
+        _PENALTIES = _penalties_function()
+    flat = theta.reshape(-1, 2).to(cs.device, torch.float64)
+    if flat.shape[0] > native.CALIB_FOLD_ROWS:
+        g, c = cs.position_params(theta)
+    else:
+        g, c = _PENALTIES.apply(flat, cs, engine)
     return _FN.apply(g, c, cs, engine, precision)
 
 

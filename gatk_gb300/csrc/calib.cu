@@ -425,6 +425,63 @@ __global__ void __launch_bounds__(kCalibBlock) calib_kernel(DevTables TB, ghmm_c
     }
 }
 
+// Position penalties from the table: one pass over the index (8 bytes in, 8 out a position).
+__global__ void __launch_bounds__(256) calib_gather_kernel(const double *table, int64_t rows, const int64_t *index,
+                                                           int64_t n, double fixed_open, double fixed_cont,
+                                                           float *gap_open, float *gap_cont) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = index[i];
+        double g = fixed_open, c = fixed_cont;
+        if (k >= 0) {
+            g = k < rows ? __ldg(table + 2 * k) : nan("");
+            c = k < rows ? __ldg(table + 2 * k + 1) : nan("");
+        }
+        gap_open[i] = (float)g;
+        gap_cont[i] = (float)c;
+    }
+}
+
+// The gradient of the table: position gradients summed by table row, in FP64.  Most positions share a few rows (no
+// repeat, or a short one), so atomics per position queue up on a few addresses: two indexed adds of 614,000 positions
+// took 0.35 ms each that way.  Here a warp adds up the positions of each row it meets before one atomic into
+// the block's table in shared memory, and the tables are added up at the end: one pass over 16 bytes a position.
+__global__ void __launch_bounds__(256) calib_fold_kernel(const int64_t *index, int64_t n, const float *grad_open,
+                                                         const float *grad_cont, int rows, double *table) {
+    extern __shared__ double fold_tab[];
+    for (int t = threadIdx.x; t < 2 * rows; t += blockDim.x) fold_tab[t] = 0.0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < n; base += warps * 32) {
+        const int64_t i = base + lane;
+        const int64_t at = i < n ? index[i] : -1;
+        const int key = at >= 0 && at < rows ? (int)at : -1;
+        const double o = key >= 0 ? (double)grad_open[i] : 0.0, c = key >= 0 ? (double)grad_cont[i] : 0.0;
+        unsigned todo = __ballot_sync(kFullMask, key >= 0);
+        while (todo) {  // one table row a round
+            const int first = __ffs(todo) - 1;
+            const int row = __shfl_sync(kFullMask, key, first);
+            const unsigned same = __ballot_sync(kFullMask, key == row);
+            double so = key == row ? o : 0.0, sc = key == row ? c : 0.0;
+            if (same & (same - 1)) {
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) {
+                    so += __shfl_xor_sync(kFullMask, so, d);
+                    sc += __shfl_xor_sync(kFullMask, sc, d);
+                }
+            }
+            if (lane == first) {
+                atomicAdd(&fold_tab[2 * row], so);
+                atomicAdd(&fold_tab[2 * row + 1], sc);
+            }
+            todo &= ~same;
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 2 * rows; t += blockDim.x)
+        if (fold_tab[t] != 0.0) atomicAdd(table + t, fold_tab[t]);
+}
+
 // Blocks of one instantiation resident on an SM (from its registers), looked up once per process.
 template <typename T, int K, bool BACKWARD, bool MULTI>
 int calib_resident_blocks() {
@@ -499,6 +556,20 @@ int launch_calib(const DevTables &TB, const ghmm_calib_batch &in, int k, bool ba
     }
 #undef GHMM_CALIB
 #undef GHMM_CALIB_ONE
+    return (int)cudaGetLastError();
+}
+
+int launch_calib_gather(const double *table, int64_t rows, const int64_t *index, int64_t n, double fixed_open,
+                        double fixed_cont, float *gap_open, float *gap_cont, int sm_count, cudaStream_t s) {
+    const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count * 8);
+    calib_gather_kernel<<<grid, 256, 0, s>>>(table, rows, index, n, fixed_open, fixed_cont, gap_open, gap_cont);
+    return (int)cudaGetLastError();
+}
+
+int launch_calib_fold(const int64_t *index, int64_t n, const float *grad_open, const float *grad_cont, int rows,
+                      double *table, int sm_count, cudaStream_t s) {
+    const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count * 2);
+    calib_fold_kernel<<<grid, 256, 2 * (size_t)rows * sizeof(double), s>>>(index, n, grad_open, grad_cont, rows, table);
     return (int)cudaGetLastError();
 }
 

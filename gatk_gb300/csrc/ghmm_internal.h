@@ -167,6 +167,10 @@ int calib_block();
 int launch_calib(const DevTables &TB, const ghmm_calib_batch &in, int k, bool backward, bool fp64, void *scratch,
                  int64_t scratch_bytes_per_warp, double *loglik, const double *weights, float *grad_open,
                  float *grad_cont, int *need_fp64, int grid, int sm_count, cudaStream_t s);
+int launch_calib_gather(const double *table, int64_t rows, const int64_t *index, int64_t n, double fixed_open,
+                        double fixed_cont, float *gap_open, float *gap_cont, int sm_count, cudaStream_t s);
+int launch_calib_fold(const int64_t *index, int64_t n, const float *grad_open, const float *grad_cont, int rows,
+                      double *table, int sm_count, cudaStream_t s);
 // Smith-Waterman (sw.cu).  Overhang strategies (SWOverhangStrategy) and BAM cigar op codes.
 constexpr int kSwSoftclip = 0, kSwIndel = 1, kSwLeadingIndel = 2, kSwIgnore = 3;
 constexpr uint32_t kSwOpM = 0, kSwOpI = 1, kSwOpD = 2, kSwOpS = 4;

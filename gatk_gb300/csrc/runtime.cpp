@@ -604,6 +604,34 @@ int ghmm_calib_backward(ghmm_ctx *ctx, const ghmm_calib_batch *batch, int32_t pr
     return calib_run(ctx, batch, precision, d_weights, d_loglik, d_grad_open, d_grad_cont, true);
 }
 
+int ghmm_calib_gather(ghmm_ctx *ctx, const double *d_table, int64_t rows, const int64_t *d_index, int64_t n,
+                      double fixed_open, double fixed_cont, float *d_gap_open, float *d_gap_cont, void *stream) {
+    if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
+    if (n < 0 || rows < 0) return fail(ctx, GHMM_ERR_ARG, "negative size");
+    if (n == 0) return GHMM_OK;
+    if (!d_index || !d_gap_open || !d_gap_cont || (rows > 0 && !d_table)) return fail(ctx, GHMM_ERR_ARG, "NULL argument");
+    GHMM_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
+    const int e = launch_calib_gather(d_table, rows, d_index, n, fixed_open, fixed_cont, d_gap_open, d_gap_cont,
+                                      ctx->sm_count, (cudaStream_t)stream);
+    if (e) return cuda_fail(ctx, (cudaError_t)e, "calibration gather launch");
+    return GHMM_OK;
+}
+
+int ghmm_calib_fold(ghmm_ctx *ctx, const int64_t *d_index, int64_t n, const float *d_grad_open,
+                    const float *d_grad_cont, int64_t rows, double *d_table, void *stream) {
+    if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
+    if (n < 0 || rows < 0 || rows > GHMM_CALIB_FOLD_ROWS) return fail(ctx, GHMM_ERR_ARG, "size out of range");
+    if (rows == 0) return GHMM_OK;
+    if (!d_table || (n > 0 && (!d_index || !d_grad_open || !d_grad_cont))) return fail(ctx, GHMM_ERR_ARG, "NULL argument");
+    GHMM_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
+    GHMM_CUDA(cudaMemsetAsync(d_table, 0, (size_t)rows * 2 * sizeof(double), (cudaStream_t)stream), "clear table gradient");
+    if (n == 0) return GHMM_OK;
+    const int e = launch_calib_fold(d_index, n, d_grad_open, d_grad_cont, (int)rows, d_table, ctx->sm_count,
+                                    (cudaStream_t)stream);
+    if (e) return cuda_fail(ctx, (cudaError_t)e, "calibration fold launch");
+    return GHMM_OK;
+}
+
 int ghmm_measure_peaks(ghmm_ctx *ctx, double *fp32, double *fp32x2, double *fp64) {
     if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
     double a = 0, b = 0, c = 0;

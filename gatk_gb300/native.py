@@ -28,6 +28,7 @@ MODE_PD = 3
 MODE_PD_FP32 = 4
 INJECT_REFUSE_ALLOCATIONS = 1
 INJECT_FP64_RERUN_EVERY = 2
+CALIB_FOLD_ROWS = 2048  # GHMM_CALIB_FOLD_ROWS
 FP64_RESCALED_FLOOR = -560.0  # GHMM_FP64_RESCALED_FLOOR
 MODE_PLAIN_FP64 = 2
 
@@ -253,6 +254,11 @@ _SIGS = {
     "ghmm_debug_pd_ops": (ctypes.c_int, [_u8p, _u8p, ctypes.c_int32, _u8p, _u8p]),
     "ghmm_debug_pipeline_cuts": (ctypes.c_int, [_i64p, ctypes.c_int64, _i64p, ctypes.c_int64, _i64p]),
     "ghmm_str_analyze": (ctypes.c_int, [_u8p, ctypes.c_int32, ctypes.c_int32, _i32p, _i32p, _i32p]),
+    "ghmm_calib_gather": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+                                         ctypes.c_int64, ctypes.c_double, ctypes.c_double, ctypes.c_void_p,
+                                         ctypes.c_void_p, ctypes.c_void_p]),
+    "ghmm_calib_fold": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+                                       ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]),
     "ghmm_calib_forward": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(CalibBatch), ctypes.c_int32, ctypes.c_void_p]),
     "ghmm_calib_backward": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(CalibBatch), ctypes.c_int32, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),

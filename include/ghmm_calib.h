@@ -58,6 +58,17 @@ int ghmm_calib_forward(ghmm_ctx *ctx, const ghmm_calib_batch *batch, int32_t pre
 int ghmm_calib_backward(ghmm_ctx *ctx, const ghmm_calib_batch *batch, int32_t precision, const double *d_weights,
                         double *d_loglik, float *d_grad_open, float *d_grad_cont);
 
+/* Gap penalties per read position from a table of (gap open, gap continuation) rows, and the gradient back into it
+ * (device arrays, enqueued on `stream`, a cudaStream_t, without waiting).  index[p] is position p's table row, or < 0 for
+ * a position with the fixed penalties fixed_open / fixed_cont (it adds nothing to the gradient); rows outside the table
+ * give NaN.  ghmm_calib_fold sums the float gradients in FP64 into d_table[2 * rows], which it first clears;
+ * rows <= GHMM_CALIB_FOLD_ROWS. */
+#define GHMM_CALIB_FOLD_ROWS 2048
+int ghmm_calib_gather(ghmm_ctx *ctx, const double *d_table, int64_t rows, const int64_t *d_index, int64_t n,
+                      double fixed_open, double fixed_cont, float *d_gap_open, float *d_gap_cont, void *stream);
+int ghmm_calib_fold(ghmm_ctx *ctx, const int64_t *d_index, int64_t n, const float *d_grad_open,
+                    const float *d_grad_cont, int64_t rows, double *d_table, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
