@@ -69,3 +69,25 @@ def test_results_do_not_depend_on_the_task_split():
     finally:
         eng.close()
     assert np.array_equal(np.concatenate(alone), together[:sum(len(a) for a in alone)])
+
+
+def test_short_haplotype_in_a_task_changes_no_other_result():
+    """A haplotype of fewer than 63 columns sends its task's steps through the checked form; the other haplotypes' results
+    keep every bit, at the lengths around that limit, in one and several strips."""
+    rng = np.random.default_rng(13)
+    region = _region(rng, [2, 30, 31, 62, 94, 126, 158, 190, 222, 254, 300, 520, 521] + list(range(60, 200, 3)),
+                     [63, 64, 65, 126, 127, 200, 90])
+    short = _region(rng, [1], [62, 1, 40])[0]
+    haps, reads = region
+    out = {}
+    eng = Engine()
+    try:
+        for name, hs in (("long", haps), ("mixed", [short[0]] + haps[:3] + [short[1]] + haps[3:] + [short[2]])):
+            with eng.batch(workload.from_pairs([(hs, reads)] * 256)) as b:  # enough work for whole regions a task
+                b.forward(native.MODE_FP32_RERUN)
+                out[name] = b.results().reshape(256, len(reads), len(hs))
+    finally:
+        eng.close()
+    assert np.array_equal(out["mixed"][:, :, [1, 2, 3, 5, 6, 7, 8]], out["long"])
+    want = oracle.compute_workload(workload.from_pairs([(haps, reads)])).reshape(len(reads), len(haps))
+    assert np.abs(out["long"] - want).max() <= 1e-3
