@@ -16,7 +16,7 @@
 // the backward runs the strips last to first, and the adjoint values a strip's first row hands the row above are
 // kept in scratch per column for the strip above it.
 //  * Forward: the whole warp front (each lane's K rows of M, I, D plus the diagonal inputs) is saved to scratch
-//    every kSeg steps (the checkpoints); lane 31 sums the last row into L_s (scaled likelihood).
+//    every kSeg (8) steps (the checkpoints); lane 31 sums the last row into L_s (scaled likelihood).
 //  * Backward: segments are processed last to first.  Each segment's forward is recomputed from its checkpoint,
 //    keeping every step's front, and then the adjoint wavefront runs over it in reverse: lane l at reverse step s
 //    handles column s - l, receiving from lane l+1 (the row below) by __shfl_down_sync.  Adjoints are seeded with
@@ -31,6 +31,7 @@
 #include <atomic>
 #include <cfloat>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/ghmm.h"
 #include "../../include/ghmm_calib.h"
@@ -40,7 +41,11 @@ namespace ghmm {
 namespace {
 
 constexpr unsigned kFullMask = 0xffffffffu;
-constexpr int kSeg = 16;  // steps between checkpoints (and per recomputed segment)
+// Steps between checkpoints (and per recomputed segment).  Eight: the segments of an SM's 12 warps (20 KB each at K = 5)
+// then nearly fit its L1, and the checkpoints (2.5 KB a segment and warp) stay a minor stream.  Backward of 4,096 pairs
+// of 150 x 300 bases: 855 us at 16, 810 at 8, 815 at 6, 855 at 4; of 8,345 pairs of up to 250 x 600: 3,113, 2,994,
+// 3,058, 3,149 (both at 16 with fronts of single values and each loaded twice: 854 and 3,588).
+constexpr int kSeg = 8;
 constexpr int kCalibBlock = 64;
 
 template <typename T>
@@ -168,31 +173,73 @@ __device__ __forceinline__ void fwd_step(const Rows<T, K> &w, Front<T, K> &f, co
     f.gD = uD;
 }
 
-// scratch layout per warp (all T): checkpoints [nck][3K+3][32], segment fronts [kSeg][3K+3][32], the strips' last
+// A front in scratch: 3 K + 3 values a lane, in 16-byte vectors [vector][lane] (18 values at K = 5: 5 vector accesses
+// instead of 18).
+template <typename T>
+struct Vec16;
+template <>
+struct Vec16<float> {
+    using type = float4;
+    static constexpr int n = 4;
+};
+template <>
+struct Vec16<double> {
+    using type = double2;
+    static constexpr int n = 2;
+};
+template <typename T, int K>
+constexpr int kFrontSize = (3 * K + 3 + Vec16<T>::n - 1) / Vec16<T>::n * Vec16<T>::n;  // values a lane, whole vectors
+
+// scratch layout per warp (all T): checkpoints [nck][front][32], segment fronts [kSeg][front][32], the strips' last
 // rows [nstrips - 1][H][3] (forward), and two buffers [H][4] of first-row adjoint values (backward, by strip parity)
 template <typename T, int K>
 __device__ __forceinline__ void save_front(T *dst, const Front<T, K> &f, int lane) {
+    constexpr int N = Vec16<T>::n, F = kFrontSize<T, K>;
+    T v[F];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        dst[(3 * k + 0) * 32 + lane] = f.M[k];
-        dst[(3 * k + 1) * 32 + lane] = f.I[k];
-        dst[(3 * k + 2) * 32 + lane] = f.D[k];
+        v[3 * k + 0] = f.M[k];
+        v[3 * k + 1] = f.I[k];
+        v[3 * k + 2] = f.D[k];
     }
-    dst[(3 * K + 0) * 32 + lane] = f.gM;
-    dst[(3 * K + 1) * 32 + lane] = f.gI;
-    dst[(3 * K + 2) * 32 + lane] = f.gD;
+    v[3 * K + 0] = f.gM;
+    v[3 * K + 1] = f.gI;
+    v[3 * K + 2] = f.gD;
+#pragma unroll
+    for (int i = 3 * K + 3; i < F; ++i) v[i] = (T)0;
+    auto *out = reinterpret_cast<typename Vec16<T>::type *>(dst) + lane;
+#pragma unroll
+    for (int i = 0; i < F / N; ++i) {
+        if constexpr (N == 4)
+            out[i * 32] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        else
+            out[i * 32] = make_double2(v[2 * i], v[2 * i + 1]);
+    }
 }
 template <typename T, int K>
 __device__ __forceinline__ void load_front(const T *src, Front<T, K> &f, int lane) {
+    constexpr int N = Vec16<T>::n, F = kFrontSize<T, K>;
+    T v[F];
+    const auto *in = reinterpret_cast<const typename Vec16<T>::type *>(src) + lane;
+#pragma unroll
+    for (int i = 0; i < F / N; ++i) {
+        const auto x = in[i * 32];
+        v[N * i] = x.x;
+        v[N * i + 1] = x.y;
+        if constexpr (N == 4) {
+            v[N * i + 2] = x.z;
+            v[N * i + 3] = x.w;
+        }
+    }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        f.M[k] = src[(3 * k + 0) * 32 + lane];
-        f.I[k] = src[(3 * k + 1) * 32 + lane];
-        f.D[k] = src[(3 * k + 2) * 32 + lane];
+        f.M[k] = v[3 * k + 0];
+        f.I[k] = v[3 * k + 1];
+        f.D[k] = v[3 * k + 2];
     }
-    f.gM = src[(3 * K + 0) * 32 + lane];
-    f.gI = src[(3 * K + 1) * 32 + lane];
-    f.gD = src[(3 * K + 2) * 32 + lane];
+    f.gM = v[3 * K + 0];
+    f.gI = v[3 * K + 1];
+    f.gD = v[3 * K + 2];
 }
 
 // MULTI: reads may need more than one strip (K = 8 batches with reads longer than 256 bases); otherwise every read fits
@@ -200,7 +247,7 @@ __device__ __forceinline__ void load_front(const T *src, Front<T, K> &f, int lan
 template <typename T, int K, bool BACKWARD, bool MULTI>
 __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int64_t pair, T *scratch, double *loglik,
                            const double *weights, float *grad_open, float *grad_cont, int *need_fp64, bool fp64_pass) {
-    constexpr int F = 3 * K + 3;  // values per lane in a front
+    constexpr int F = kFrontSize<T, K>;  // values per lane in a front
     const int lane = threadIdx.x & 31;
     const int read = in.pair_read[pair], hap = in.pair_hap[pair];
     const int64_t roff = in.read_off[read];
@@ -291,6 +338,7 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
         T dgA = (T)0, dgB = (T)0;  // from the row below: a*gamma, b*gamma of its first row at column c+1
         T snA = (T)0, snB = (T)0, snE = (T)0, snF = (T)0;  // what this lane sent last reverse step
         const bool below = lane != 31 || !last;  // lane 31 of the last strip holds the read's last row
+        Front<T, K> cur;  // the front after the step being reversed
         for (int sg = nseg - 1; sg >= 0; --sg) {
             const int s0 = sg * kSeg, s1 = min(s0 + kSeg, nsteps);
             // recompute the segment's fronts (front after each step, plus the step's "up" values)
@@ -302,10 +350,13 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
                 T *dst = seg + (size_t)(s - s0) * F * 32;
                 save_front<T, K>(dst, r, lane);  // gM/gI/gD slots now hold this step's up values
             }
+            if (sg == nseg - 1) cur = r;
             __syncwarp();
-            for (int s = s1 - 1; s >= s0; --s) {
+            // One reverse step.  ALL: every lane's column is inside the haplotype (all but the first and last 31 steps).
+            auto reverse_step = [&](const int s, auto all_tag) {
+                constexpr bool ALL = decltype(all_tag)::value;
                 const int c = s - lane;
-                const bool valid = c >= 0 && c < H;
+                const bool valid = ALL || (c >= 0 && c < H);
                 // below (row under this lane's last row) at column c, and its a*gamma, b*gamma for column c: from
                 // lane l+1, or for lane 31 from the first row of the strip below
                 T inE = __shfl_down_sync(kFullMask, snE, 1), inF = __shfl_down_sync(kFullMask, snF, 1);
@@ -317,16 +368,11 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
                     inA = have ? adj_in[4 * c + 2] : (T)0;
                     inB = have ? adj_in[4 * c + 3] : (T)0;
                 }
-                // forward values: column c (after step s) and c-1 (after step s-1)
-                Front<T, K> cur, prv;
-                load_front<T, K>(seg + (size_t)(s - s0) * F * 32, cur, lane);
-                if (s > s0) {
-                    load_front<T, K>(seg + (size_t)(s - 1 - s0) * F * 32, prv, lane);
-                } else {
-                    load_front<T, K>(scratch + (size_t)sg * F * 32, prv, lane);  // checkpoint = front before step s0
-                    // the checkpoint's gM/gI/gD are the diagonal inputs of step s0 = up values of step s0-1
-                }
-                if (c == 0) {  // the forward used the column-0 boundary as left and diagonal inputs here
+                // forward values: column c (cur, after step s) and c-1 (after step s-1; the checkpoint is the front before
+                // step s0, its gM/gI/gD the up values of step s0-1)
+                Front<T, K> prv;
+                load_front<T, K>(s > s0 ? seg + (size_t)(s - 1 - s0) * F * 32 : scratch + (size_t)sg * F * 32, prv, lane);
+                if ((!ALL || s < 32) && c == 0) {  // the forward used the column-0 boundary as left and diagonal inputs here
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
                         prv.M[k] = prv.I[k] = (T)0;
@@ -338,7 +384,7 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
                 // up values of step s (row above at column c) and diagonal (column c-1)
                 const T upM = cur.gM, upI = cur.gI;
                 const T dgM = prv.gM, dgI = prv.gI, dgD = prv.gD;
-                const uint32_t y = valid ? (uint32_t)hb[c] : 0x200u;
+                const uint32_t y = ALL || valid ? (uint32_t)hb[c] : 0x200u;
                 const bool last_lane = lane == 31;
                 T newGam[K], newBI[K], newBD[K];
                 T belowE = below ? inE : (T)0, belowF = below ? inF : (T)0;  // e,f of row below times its betaI
@@ -353,7 +399,7 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
                     const T pr = prior_of<T>(w.rb[k], y, w.pm[k], w.pe[k]);
                     T g = pr * bM;
                     T bi = bI_new, bd = bD_new;
-                    if (!valid) g = bi = bd = (T)0;
+                    if (!ALL && !valid) g = bi = bd = (T)0;
                     newGam[k] = g;
                     newBI[k] = bi;
                     newBD[k] = bd;
@@ -391,6 +437,13 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
                 }
                 dgA = inA;  // the row below's a*gamma at column c becomes the diagonal input of column c-1
                 dgB = inB;
+                cur = prv;  // also into the next segment: its last front is this one's checkpoint
+            };
+            for (int s = s1 - 1; s >= s0; --s) {
+                if (s >= 31 && s < H)
+                    reverse_step(s, std::true_type{});
+                else
+                    reverse_step(s, std::false_type{});
             }
             __syncwarp();
         }
@@ -409,8 +462,16 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
     }
 }
 
+// Blocks an SM that ptxas is asked to fit (0: as it likes).  The FP32 backward of up to 160 rows at six, three warps a
+// scheduler: left alone it takes more than 168 registers and fits five (4,096 pairs: 976 against 855 us), and seven
+// blocks need 128 registers, since warps are allotted registers per scheduler, and spill (1,133 us).
+template <typename T, int K, bool BACKWARD>
+struct CalibMinBlocks {
+    static constexpr int value = sizeof(T) == 4 && BACKWARD && K <= 5 ? 6 : 0;
+};
+
 template <typename T, int K, bool BACKWARD, bool MULTI>
-__global__ void __launch_bounds__(kCalibBlock) calib_kernel(DevTables TB, ghmm_calib_batch in, T *scratch,
+__global__ void __launch_bounds__(kCalibBlock, CalibMinBlocks<T, K, BACKWARD>::value) calib_kernel(DevTables TB, ghmm_calib_batch in, T *scratch,
                                                             int64_t scratch_per_warp, double *loglik,
                                                             const double *weights, float *grad_open, float *grad_cont,
                                                             int *need_fp64, int fp64_pass) {
@@ -500,18 +561,17 @@ int calib_resident_blocks() {
 }  // namespace
 
 int64_t calib_scratch_per_warp(int k, int max_hap_len, int max_read_len, bool fp64) {
-    const int64_t F = 3 * k + 3;
+    const int64_t vec = fp64 ? 2 : 4, F = (3 * k + 3 + vec - 1) / vec * vec;
     const int64_t nsteps = max_hap_len + 31;
     const int64_t fronts = (nsteps + kSeg - 1) / kSeg + kSeg;
     const int64_t nstrips = ((int64_t)max_read_len + 32 * k - 1) / (32 * k);
     const int64_t boundaries = (nstrips - 1) * max_hap_len * 3 + 2 * (int64_t)max_hap_len * 4;
-    return (fronts * F * 32 + boundaries) * (fp64 ? 8 : 4);
+    return (fronts * F * 32 + boundaries + 3) / 4 * 4 * (fp64 ? 8 : 4);  // whole 16-byte vectors
 }
 
-// Six blocks of two warps per SM: 12 warps, what the 154-register FP32 backward at K = 5 keeps resident; on
-// 4,096 pairs of 150-base reads and 300-base haplotypes 7 % faster forward + backward than four blocks, and
-// faster than eight.  Instantiations
-// with fewer resident blocks (the FP64 backward at up to 255 registers) launch only those, so that no block waits
+// Six blocks of two warps per SM: 12 warps, what the FP32 backward at K = 5 keeps resident; on 4,096 pairs of
+// 150-base reads and 300-base haplotypes 7 % faster forward + backward than four blocks, and faster than eight.
+// Instantiations with fewer resident blocks (the FP64 backward at up to 255 registers) launch only those, so that no block waits
 // for a second wave with pairs already assigned to it by the grid stride.
 int calib_grid(int sm_count) { return sm_count * 6; }
 int calib_block() { return kCalibBlock; }
