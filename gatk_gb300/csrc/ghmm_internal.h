@@ -109,6 +109,7 @@ struct PdPlanes {
     const uint8_t *flags;
     const uint8_t *states;
     const uint8_t *ops;  // per column the packed FP32 kernel's op byte, indexed like hap_code (kCodePad zeros around)
+    const uint8_t *snps; // per column the SNP bits of the op byte, also where the column goes through the prior table
 };
 // Op bits of the packed FP32 PD kernel (pd_packed.cu), derived per haplotype column by the host (pd_host.cpp).
 constexpr uint32_t kPdOpCopy = 1;       // a later column reads this column's branch state: store it (NORMAL: bX =
@@ -118,9 +119,16 @@ constexpr uint32_t kPdOpDelEnd = 4;     // DEL_END column: I reads max(bX, X) of
 constexpr uint32_t kPdOpNextAfter = 8;  // the next column is AFTER_DEL
 constexpr uint32_t kPdOpSnp = 16;       // undetermined SNP: its alternative in bits 5-6 (A, C, G, T = 0..3)
 constexpr int kPdOpAltShift = 5;
+// PD column codes: base index kPdSlotBase marks an undetermined SNP column whose priors the packed kernel keeps in its
+// table, with the column's base in bits 3-4 and no SNP bits in its op byte; at least kPdSlotGap columns after the last one
+// of its region, so that the last lane has passed that one when the first lane meets the next.
+constexpr uint32_t kPdSlotBase = 5;
+constexpr int kPdSlotRefShift = 3;
+constexpr int kPdSlotGap = 63;
+constexpr uint32_t kPdOpSnpBits = 16 | 3 << kPdOpAltShift | 128;
 constexpr uint32_t kPdOpSnpAllBut = 128;  // with kPdOpSnp: three bases match, bits 5-6 name the fourth
 // FP32 PD read-pair tasks of bucket key (2..8 rows per lane, | 16 for multi-strip tasks) from the batch's task list.
-int launch_pd_bucket(const DevTables &t, const DevBatch &b, const uint8_t *ops, int key, int grid, cudaStream_t s);
+int launch_pd_bucket(const DevTables &t, const DevBatch &b, const PdPlanes &pd, int key, int grid, cudaStream_t s);
 int pd_bucket_occupancy(int key, int *blocks_per_sm);
 int pd_kernel_occupancy(int *blocks_per_sm);
 // PD pairs [begin, begin + count) of the pair list (count_dev: the count in device memory), K rows per lane, in

@@ -140,12 +140,13 @@ int pd_marshal(ghmm_ctx *ctx, const ghmm_pd_region *regs, int64_t G, ghmm_batch 
     int rc = batch_marshal(ctx, src, b);
     if (rc) return rc;
     const int64_t NH = b.n_haps, HB = b.hap_bytes;
-    // flags | states | kCodePad zeros | ops | kCodePad zeros
-    const int64_t pd_bytes = 3 * HB + 2 * kCodePad;
+    // flags | states | kCodePad zeros | ops | kCodePad zeros | SNP bits
+    const int64_t pd_bytes = 4 * HB + 2 * kCodePad;
     GHMM_CUDA(b.h_pd.reserve((size_t)pd_bytes), "pinned PD planes");
     const int64_t *o = b.h_off.p;
     const int64_t *hap_off = o + b.n_reads + 1;
     uint8_t *flags = b.h_pd.p, *states = b.h_pd.p + HB, *ops = b.h_pd.p + 2 * HB + kCodePad;
+    uint8_t *snps = ops + HB + kCodePad;
     memset(ops - kCodePad, 0, (size_t)kCodePad);
     memset(ops + HB, 0, (size_t)kCodePad);
     const uint8_t *hraw = b.h_hap.p;
@@ -162,6 +163,19 @@ int pd_marshal(ghmm_ctx *ctx, const ghmm_pd_region *regs, int64_t G, ghmm_batch 
         for (int j = 0; j < H; j++)
             if (flags[a + j] & 4) code[j] |= 16;
         pd_ops(flags + a, hraw + a, code, H, ops + a, hcode + a);
+    });
+    // undetermined SNP columns far enough behind one another go through the packed kernel's prior table (kPdSlotBase)
+    const int64_t *rho_slots = o + b.n_reads + 1 + NH + 1 + G + 1;
+    parallel_for(G, hw_threads(ctx->max_threads), [&](int64_t g) {
+        const int64_t first = hap_off[rho_slots[g]], end = hap_off[rho_slots[g + 1]];
+        int64_t free_from = first;
+        for (int64_t j = first; j < end; j++) {
+            snps[j] = ops[j] & kPdOpSnpBits;
+            if (!(ops[j] & kPdOpSnp) || j < free_from) continue;
+            free_from = j + kPdSlotGap;
+            ops[j] &= (uint8_t)~kPdOpSnpBits;
+            hcode[j] = (uint8_t)((hcode[j] & (kColFirst | kColLast)) | kPdSlotBase | ((hcode[j] & 3u) << kPdSlotRefShift));
+        }
     });
     // a read base outside ACGTacgtN that meets an undetermined SNP column throws in the reference
     const int64_t *rro = o + b.n_reads + 1 + NH + 1, *rho = rro + G + 1;
@@ -184,12 +198,13 @@ int pd_marshal(ghmm_ctx *ctx, const ghmm_pd_region *regs, int64_t G, ghmm_batch 
 int pd_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s) {
     int rc = batch_upload(ctx, b, s);
     if (rc) return rc;
-    const int64_t HB = b.hap_bytes, pd_bytes = 3 * HB + 2 * kCodePad;
+    const int64_t HB = b.hap_bytes, pd_bytes = 4 * HB + 2 * kCodePad;
     GHMM_CUDA(b.d_pd.reserve((size_t)pd_bytes), "device PD planes");
     GHMM_CUDA(cudaMemcpyAsync(b.d_pd.p, b.h_pd.p, (size_t)pd_bytes, cudaMemcpyHostToDevice, s), "H2D PD planes");
     b.pd.flags = b.d_pd.p;
     b.pd.states = b.d_pd.p + HB;
     b.pd.ops = b.d_pd.p + 2 * HB + kCodePad;
+    b.pd.snps = b.pd.ops + HB + kCodePad;
     b.upload_bytes += pd_bytes;
     return GHMM_OK;
 }
@@ -293,7 +308,7 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s) 
                     const int64_t want = (bk.count + kWarpsPerBlock - 1) / kWarpsPerBlock;
                     int g = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * bp));
                     if (bk.key & 16) g = std::min(g, bk.grid);  // the strip scratch is sized for the regular kernel's grid
-                    const int e = launch_pd_bucket(ctx->tables, d, b.pd.ops, bk.key, g, st);
+                    const int e = launch_pd_bucket(ctx->tables, d, b.pd, bk.key, g, st);
                     return e ? cuda_fail(ctx, (cudaError_t)e, "PD-HMM packed launch") : GHMM_OK;
                 });
             });

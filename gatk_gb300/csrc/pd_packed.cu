@@ -25,12 +25,18 @@
 //    applies the max in its hand-over at this column.
 //  * kPdOpNextAfter: the next column is AFTER_DEL, so the lane's hand-over of row 0's M~ inner sum for it (the
 //    lane below's diagonal input there) uses max(bX, X) of its last row.
-//  * kPdOpSnp (alternative base in bits 5-6): the prior is the match prior when the read base equals the column's
+//  * An SNP column far enough behind the last one of its region (kPdSlotGap) has no op at all: when lane 0 meets it, all
+//    lanes compute their rows' priors for it once, into a row of the prior table that its column code names, and the step
+//    of every lane reads that row as it reads a base's.  (As an op it would cost 32 steps in each of which one lane does
+//    that work alone.)
+//  * kPdOpSnp (alternative base in bits 5-6), on the others: the prior is the match prior when the read base equals the column's
 //    base or the alternative (or is N), picked from three rows of the prior table without a per-row base compare;
 //    with kPdOpSnpAllBut, three bases match (two alternatives) and bits 5-6 name the fourth.  A column whose
 //    alternatives cover all four bases carries the code of N (pd_host.cpp), which matches every read base.
 // These run only in lanes at such columns (lane-divergent branches), and only in steps where some lane of the warp
-// is at such a column (a warp vote; the other steps are the regular kernel's).  The accumulator rows below each read
+// is at such a column (a warp vote; the other steps are the regular kernel's).  From the last column with an op until 62
+// steps later steps vote; beyond, up to the next one (found by scanning the op plane), they are the regular kernel's
+// without a vote, unrolled.  The accumulator rows below each read
 // never take a branch state (theirs stay 0, so max(bX, X) = X for them), and the first accumulator row's I never
 // takes the DEL_END max, since it sums the read's last row rather than stepping the recurrence.
 //
@@ -89,6 +95,8 @@ __device__ __forceinline__ void emit_pd(const DevBatch &B, float t, float2 scale
     }
 }
 
+constexpr int kOpFree = 0, kOps = 1, kCheck = 2;  // kinds of wavefront steps
+
 // Blocks of 128 threads per SM ptxas is asked to fit: the branch registers (six floats per row) on top of the
 // regular kernel's.
 template <int K>
@@ -98,7 +106,8 @@ struct PdMinBlocks {
 
 template <int K, bool MULTI>
 __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(DevTables T, DevBatch B,
-                                                                             const uint8_t *ops_plane) {
+                                                                             const uint8_t *ops_plane,
+                                                                             const uint8_t *snp_plane) {
     static_assert(K >= 2, "the accumulator rows need two rows of lane 31");
     constexpr int KEY = K | (MULTI ? 16 : 0);
     constexpr int S = 32 * K;
@@ -106,11 +115,12 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
     const int counter_slot = kCounterBucketBase + KEY;
     const int lane = threadIdx.x & 31;
     constexpr int KP = (K + 1) / 2;  // row pairs of the prior table
+    constexpr int kRows = kBases + 1;  // prior rows per row pair: the bases, and the SNP column of the moment (kPdSlot)
     extern __shared__ float4 pd_prior_smem4[];
-    float4 *prior_tbl4 = pd_prior_smem4 + (size_t)(threadIdx.x >> 5) * (KP * kBases * 32) + lane;
+    float4 *prior_tbl4 = pd_prior_smem4 + (size_t)(threadIdx.x >> 5) * (KP * kRows * 32) + lane;
     float2 *prior_tbl2 = reinterpret_cast<float2 *>(prior_tbl4);
     // branch states bM, bI, bD of the lane's rows, lane-private: [row][M, I, D][lane] after the 4 warps' tables
-    float2 *bst = reinterpret_cast<float2 *>(pd_prior_smem4 + 4 * (KP * kBases * 32)) +
+    float2 *bst = reinterpret_cast<float2 *>(pd_prior_smem4 + 4 * (KP * kRows * 32)) +
                   (size_t)(threadIdx.x >> 5) * (K * 3 * 32) + lane;
     // strip boundary of multi-strip tasks: per column lane 31's hand-over (I~ and the M~ inner sum) for lane 0 of
     // the next strip, as the regular kernel passes it
@@ -142,6 +152,7 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
         const int ncols = (int)(B.hap_off[task.hap_end] - col0);
         const uint8_t *stream = B.hap_code + col0;
         const uint8_t *opstream = ops_plane + col0;
+        const uint8_t *snps = snp_plane + col0;
         const int nstrips = MULTI ? task.nstrips : 1;
 
         for (int strip = 0; strip < nstrips; ++strip) {
@@ -161,9 +172,10 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
 #pragma unroll
                 for (int h = 0; h < kBases; ++h) {
                     const uint32_t hm = kBaseMask[h];
-                    prior_tbl2[((k / 2) * kBases + h) * 64 + (k & 1)] =
+                    prior_tbl2[((k / 2) * kRows + h) * 64 + (k & 1)] =
                         make_float2((a.code & hm) ? a.pm : a.pe, (b.code & hm) ? b.pm : b.pe);
                 }
+                prior_tbl2[((k / 2) * kRows + (int)kPdSlotBase) * 64 + (k & 1)] = zero2();
             }
             float2 b0n = shfl_down2(cb[0]), c0n = shfl_down2(cc[0]), e0n = shfl_down2(ce[0]);
             if (lane == 31) {  // the row below lane 31: the next strip's first row, or none
@@ -197,13 +209,47 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
             // code and op of the next step's column, loaded a step ahead (both planes have kCodePad zero bytes on
             // either side, so columns just outside the stream read as code 0 and no op)
             uint32_t code_next = (uint32_t)__ldg(stream - 2 * lane);
-            uint32_t op_next = (uint32_t)__ldg(opstream - 2 * lane);
-            auto step = [&](const int s, auto chk_tag) {
-                constexpr bool CHK = decltype(chk_tag)::value;
+            uint32_t op_next = 0u;
+            // the priors of row pair kk at an undetermined SNP column of base ref, from the table rows of bases
+            auto snp_row = [&](int kk, uint32_t ref, uint32_t op) -> float4 {
+                const uint32_t alt = (op >> kPdOpAltShift) & 3u;
+                const float4 *row = prior_tbl4 + kk * kRows * 32;
+                if (op & kPdOpSnpAllBut) {  // three bases match: all but `alt`
+                    const float4 tu = row[alt * 32], tn = row[4 * 32], tw = row[(alt ? 0u : 1u) * 32];
+                    return make_float4(all_but_prior(tu.x, tn.x, tw.x), all_but_prior(tu.y, tn.y, tw.y),
+                                       all_but_prior(tu.z, tn.z, tw.z), all_but_prior(tu.w, tn.w, tw.w));
+                }
+                // two bases match: the column's and `alt`
+                const uint32_t third = (uint32_t)__ffs(~((1u << ref) | (1u << alt))) - 1u;
+                const float4 t1 = row[ref * 32], t2 = row[alt * 32], t3 = row[third * 32];
+                return make_float4(snp_prior(t1.x, t2.x, t3.x), snp_prior(t1.y, t2.y, t3.y),
+                                   snp_prior(t1.z, t2.z, t3.z), snp_prior(t1.w, t2.w, t3.w));
+            };
+            // the next column from `from` on whose byte in plane, masked, lies in [low, high], or past the last step
+            auto next_column = [&](const uint8_t *plane, int from, uint32_t mask, uint32_t low, uint32_t high) -> int {
+                for (; from < ncols; from += 128) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int c = from + 32 * q + lane;
+                        const uint32_t v = c < ncols ? (uint32_t)__ldg(plane + c) & mask : 0u;
+                        const unsigned hit = __ballot_sync(kFull, v >= low && v <= high);
+                        if (hit) return from + 32 * q + __ffs(hit) - 1;
+                    }
+                }
+                return nsteps;
+            };
+            // One step.  kOpFree: no lane is at a column with PD work; kOps: some may be; kCheck: also at a first or last
+            // column, or outside the stream.
+            auto step = [&](const int s, auto kind_tag) {
+                constexpr int KIND = decltype(kind_tag)::value;
+                constexpr bool CHK = KIND == kCheck;
                 const int c = s - 2 * lane;
-                uint32_t code = code_next, op = op_next;
+                uint32_t code = code_next, op = 0u;
                 code_next = (uint32_t)__ldg(stream + c + 1);
-                op_next = (uint32_t)__ldg(opstream + c + 1);
+                if constexpr (KIND != kOpFree) {
+                    op = op_next;
+                    op_next = (uint32_t)__ldg(opstream + c + 1);
+                }
                 bool valid = true;
                 if constexpr (CHK) {
                     valid = (c >= 0) && (c < ncols);
@@ -276,35 +322,16 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
                     float2 prs[2 * KP];
 #pragma unroll
                     for (int kk = 0; kk < KP; ++kk) {
-                        const float4 v = pri4[kk * kBases * 32];
+                        const float4 v = pri4[kk * kRows * 32];
                         prs[2 * kk] = make_float2(v.x, v.y);
                         prs[2 * kk + 1] = make_float2(v.z, v.w);
                     }
                     if (OPS && (op & kPdOpSnp)) {
-                        const uint32_t alt = (op >> kPdOpAltShift) & 3u;
-                        if (op & kPdOpSnpAllBut) {  // three bases match: all but `alt`
-                            const uint32_t w = alt ? 0u : 1u;
-                            const float4 *pu = prior_tbl4 + alt * 32, *pn = prior_tbl4 + 4 * 32;
-                            const float4 *pw = prior_tbl4 + w * 32;
 #pragma unroll
-                            for (int kk = 0; kk < KP; ++kk) {
-                                const float4 tu = pu[kk * kBases * 32], tn = pn[kk * kBases * 32];
-                                const float4 tw = pw[kk * kBases * 32];
-                                prs[2 * kk] =
-                                    make_float2(all_but_prior(tu.x, tn.x, tw.x), all_but_prior(tu.y, tn.y, tw.y));
-                                prs[2 * kk + 1] =
-                                    make_float2(all_but_prior(tu.z, tn.z, tw.z), all_but_prior(tu.w, tn.w, tw.w));
-                            }
-                        } else {  // two bases match: the column's and `alt`
-                            const uint32_t third = (uint32_t)__ffs(~((1u << ref) | (1u << alt))) - 1u;
-                            const float4 *pa = prior_tbl4 + alt * 32, *pt = prior_tbl4 + third * 32;
-#pragma unroll
-                            for (int kk = 0; kk < KP; ++kk) {
-                                const float4 t2 = pa[kk * kBases * 32], t3 = pt[kk * kBases * 32];
-                                const float2 p0 = prs[2 * kk], p1 = prs[2 * kk + 1];
-                                prs[2 * kk] = make_float2(snp_prior(p0.x, t2.x, t3.x), snp_prior(p0.y, t2.y, t3.y));
-                                prs[2 * kk + 1] = make_float2(snp_prior(p1.x, t2.z, t3.z), snp_prior(p1.y, t2.w, t3.w));
-                            }
+                        for (int kk = 0; kk < KP; ++kk) {
+                            const float4 v = snp_row(kk, ref, op);
+                            prs[2 * kk] = make_float2(v.x, v.y);
+                            prs[2 * kk + 1] = make_float2(v.z, v.w);
                         }
                     }
                     // pass 1 (bottom-up): M~ and D~
@@ -366,29 +393,58 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
                 };
                 // steps where no lane is at a column with PD work (about two in three) run the regular kernel's step,
                 // without the op tests: 8 % faster than testing the op bits in every step
-                if (__any_sync(kFull, op != 0u))
-                    body(std::true_type{});
-                else
+                if constexpr (KIND == kOpFree) {
                     body(std::false_type{});
+                } else {
+                    if (__any_sync(kFull, op != 0u))
+                        body(std::true_type{});
+                    else
+                        body(std::false_type{});
+                }
             };
-            // Step loops not unrolled: the lane-divergent op branches and the two step bodies behind the warp vote
-            // split each step into several blocks anyway; unrolled 4 (checked) and 8 (check-free) the steps overflowed
-            // the instruction cache (ncu: 6-8 cycles of "no instruction" stall per issue, half the speed), and with the
-            // vote 2 (check-free) was still 4 % slower than 1
+            // Loops of steps that vote are not unrolled: the lane-divergent op branches and the two step bodies behind the
+            // vote split each step into several blocks anyway, and unrolled 4 (checked) and 8 (check-free) they overflowed
+            // the instruction cache (ncu: 6-8 cycles of "no instruction" stall per issue, half the speed).  Steps without
+            // a vote four at a time (FP32 pass of 300 regions: 11.8 ms; 1: 12.1, 2: 12.1, 8: 11.9).  Before SNP columns
+            // went through the table and stretches without ops had their own loop: 13.7 ms (the table alone: 12.6).
+            // Starts and ends of haplotypes on a known schedule, as in fp32_bucket_kernel, gained nothing here (11.7).
             const int64_t *hoff = B.hap_off + task.hap_begin;
             const int nh_task = task.hap_end - task.hap_begin;
             int s = 0, j = 0;
+            auto next_slot = [&](int from) { return next_column(stream, from, 7u, kPdSlotBase, kPdSlotBase); };
+            auto next_op = [&](int from) { return next_column(opstream, from, 255u, 1u, 255u); };
+            int slot_col = next_slot(0), op_col = next_op(0), op_until = 0;
             while (s < nsteps) {
+                if (s == slot_col) {  // lane 0 meets the column, lane 31 has passed the last one: every lane its rows' priors
+                    const uint32_t ref = ((uint32_t)__ldg(stream + s) >> kPdSlotRefShift) & 3u;
+                    const uint32_t snp = (uint32_t)__ldg(snps + s);
+#pragma unroll
+                    for (int kk = 0; kk < KP; ++kk) prior_tbl4[(kk * kRows + (int)kPdSlotBase) * 32] = snp_row(kk, ref, snp);
+                    slot_col = next_slot(s + 1);
+                }
+                if (s == op_col) {  // lane 0 meets a column with PD work, which lane 31 leaves 62 steps later
+                    op_until = s + 63;
+                    op_col = next_op(s + 1);
+                }
                 while (j <= nh_task && (int)(hoff[j] - col0) <= s) ++j;
-                const int window_end = min((int)(hoff[j - 1] - col0) + 63, nsteps);
-                if (s < window_end) {
+                const int window_end = min((int)(hoff[j - 1] - col0) + 63, nsteps), event = min(slot_col, op_col);
+                const bool check = s < window_end;
+                if (check || s < op_until) {
+                    op_next = (uint32_t)__ldg(opstream + s - 2 * lane);
+                    if (check) {
+                        const int until = min(window_end, event);
 #pragma unroll 1
-                    for (; s < window_end; ++s) step(s, std::true_type{});
+                        for (; s < until; ++s) step(s, std::integral_constant<int, kCheck>{});
+                    } else {
+                        const int until = min(min(j <= nh_task ? (int)(hoff[j] - col0) : nsteps, op_until), event);
+#pragma unroll 1
+                        for (; s < until; ++s) step(s, std::integral_constant<int, kOps>{});
+                    }
                     continue;
                 }
-                const int next_boundary = (j <= nh_task) ? (int)(hoff[j] - col0) : nsteps;
-#pragma unroll 1
-                for (; s < next_boundary; ++s) step(s, std::false_type{});
+                const int until = min(j <= nh_task ? (int)(hoff[j] - col0) : nsteps, event);
+#pragma unroll 4
+                for (; s < until; ++s) step(s, std::integral_constant<int, kOpFree>{});
             }
             if (MULTI) __syncwarp();  // the next strip's lane 0 reads what this strip's lane 31 wrote
         }
@@ -396,18 +452,18 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
 }
 
 size_t pd_bucket_smem_bytes(int k) {
-    return (size_t)(128 / 32) * (((k + 1) / 2) * kBases * 32 * sizeof(float4) + (size_t)k * 3 * 32 * sizeof(float2));
+    return (size_t)(128 / 32) * (((k + 1) / 2) * (kBases + 1) * 32 * sizeof(float4) + (size_t)k * 3 * 32 * sizeof(float2));
 }
 
 template <int K, bool MULTI>
-int launch_pd_bucket_k(const DevTables &t, const DevBatch &b, const uint8_t *ops, int grid, cudaStream_t s) {
+int launch_pd_bucket_k(const DevTables &t, const DevBatch &b, const PdPlanes &pd, int grid, cudaStream_t s) {
     const size_t smem = pd_bucket_smem_bytes(K);
     if (smem > 48 * 1024) {
         const cudaError_t e =
             cudaFuncSetAttribute(pd_bucket_kernel<K, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    pd_bucket_kernel<K, MULTI><<<grid, 128, smem, s>>>(t, b, ops);
+    pd_bucket_kernel<K, MULTI><<<grid, 128, smem, s>>>(t, b, pd.ops, pd.snps);
     return (int)cudaGetLastError();
 }
 
@@ -425,13 +481,13 @@ int pd_bucket_occupancy_k(int *blocks_per_sm) {
 }  // namespace
 
 // key: rows per lane (2..8) in the low bits, 16 for multi-strip tasks, as the regular buckets
-int launch_pd_bucket(const DevTables &t, const DevBatch &b, const uint8_t *ops, int key, int grid, cudaStream_t s) {
+int launch_pd_bucket(const DevTables &t, const DevBatch &b, const PdPlanes &pd, int key, int grid, cudaStream_t s) {
     const bool multi = (key & 16) != 0;
     switch (key & 15) {
 #define GHMM_PD_BUCKET(KK)                                                  \
     case KK:                                                                \
-        return multi ? launch_pd_bucket_k<KK, true>(t, b, ops, grid, s)     \
-                     : launch_pd_bucket_k<KK, false>(t, b, ops, grid, s);
+        return multi ? launch_pd_bucket_k<KK, true>(t, b, pd, grid, s)     \
+                     : launch_pd_bucket_k<KK, false>(t, b, pd, grid, s);
         GHMM_PD_BUCKET(2)
         GHMM_PD_BUCKET(3)
         GHMM_PD_BUCKET(4)
