@@ -137,6 +137,7 @@ struct ghmm_batch {
     int64_t pending_n_pre = 0;
     int pending_mode = -1;
     cudaGraphExec_t graph[2]{};  // captured FP32 phase (PD batches: its packed buckets) and FP64 phase
+    std::vector<unsigned char> launched_sig;  // the signature of the last forward
     std::vector<unsigned char> graph_sig;  // DevBatch bytes, mode, bucket keys and grids the graphs were captured for
 
     // bytes of the pinned and device buffers
@@ -168,6 +169,7 @@ struct ghmm_batch {
             g = nullptr;
         }
         graph_sig.clear();
+        launched_sig.clear();
         if (events_ready)
             for (auto &e : ev) cudaEventDestroy(e);
         events_ready = false;
