@@ -102,8 +102,15 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
     float4 *prior_tbl4 = prior_smem4 + (size_t)(threadIdx.x >> 5) * (KP * kBases * 32) + lane;
     float2 *prior_tbl2 = reinterpret_cast<float2 *>(prior_tbl4);
     const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    float2 *scratch = nullptr;
-    if (MULTI) scratch = B.scratch32 + warp_global * B.scratch32_cols * 3;
+    // Strip boundary (MULTI): per column lane 31's hand-over (I~, M~ inner sum) as one float4 in global scratch.  Lane 0 of
+    // the next strip reads it from a ring of 64 columns in shared memory that the warp fills 32 columns at a time, loaded
+    // 32 steps before that; read from global memory column by column, a step ahead, the load's latency was in every step
+    // (FP32 pass of reads of 510 bases x haplotypes of 600: 3,110 GCUPS, with the ring 3,845).
+    float4 *scratch = nullptr, *ring = nullptr;
+    if (MULTI) {
+        scratch = reinterpret_cast<float4 *>(B.scratch32) + warp_global * B.scratch32_cols;
+        ring = prior_smem4 + 4 * (KP * kBases * 32) + (threadIdx.x >> 5) * 64;
+    }
 
     for (;;) {
         int t = 0;
@@ -181,16 +188,32 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
             float2 pendW1 = zero2(), pendW2 = zero2();  // row 0's M~ inner sums for the next two steps
             int hap = task.hap_begin - 1;
             const bool last_strip = (strip == nstrips - 1);
-            float2 nxV = zero2(), nxW = zero2(), l0W = zero2();  // strip boundary (MULTI, lane 0): prefetched
-            if (MULTI && strip > 0 && lane == 0 && ncols > 0) {
-                nxV = scratch[0];
-                nxW = scratch[1];
+            float4 block = make_float4(0.f, 0.f, 0.f, 0.f);  // later strips: the lane's column of the ring's next 32
+            auto boundary = [&](int c) {
+                return MULTI && strip > 0 && c < ncols ? scratch[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+            };
+            float2 nxV = zero2(), nxW = zero2(), l0W = zero2();  // later strips, lane 0: the next step's entry, the last W
+            if (MULTI && strip > 0) {
+                const float4 v = boundary(lane);
+                ring[lane] = v;
+                block = boundary(32 + lane);
+                nxV = make_float2(v.x, v.y);  // (lane 0's: column 0)
+                nxW = make_float2(v.z, v.w);
             }
             float2 sV = zero2(), sW = zero2();  // what this lane hands the lane below at the end of a step
             const int nsteps = ncols + 62;
             // column code of the next step, loaded one step ahead (the code plane has kCodePad bytes on
             // both sides, so columns just outside the stream are readable; CHK steps mask them)
             uint32_t code_next = (uint32_t)__ldg(stream - 2 * lane);
+            // before the step s = 0 mod 32 of a later strip: columns s + 32 .. s + 63 into the half of the ring that columns
+            // s - 32 .. s - 1 had
+            auto refill = [&](const int s) {
+                if (!MULTI || strip == 0 || (s & 31) != 0) return;
+                __syncwarp();
+                ring[(s + 32 + lane) & 63] = block;
+                __syncwarp();
+                block = boundary(s + 64 + lane);
+            };
             // lane 31 at a haplotype's last column (K >= 2): the sums of both reads
             auto emit = [&](const int hap) {
                 const float2 t = add2(add2(Dp[K - 1], Mp[K - 1]), Ip[K >= 2 ? K - 2 : 0]);
@@ -228,11 +251,10 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
                         uV = nxV;
                         gW = l0W;
                         l0W = nxW;
-                        if (c + 1 < ncols) {
-                            nxV = scratch[2 * (c + 1) + 0];
-                            nxW = scratch[2 * (c + 1) + 1];
-                        }
                     }
+                    const float4 v = ring[(s + 1) & 63];
+                    nxV = make_float2(v.x, v.y);
+                    nxW = make_float2(v.z, v.w);
                 } else if (lane == 0) {
                     uV = zero2();
                 }
@@ -293,9 +315,8 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
                     if constexpr (CHK) {
                         if (lane == 31 && (code & kColLast)) emit(hap);
                     }
-                } else if (MULTI && lane == 31 && c >= 0 && c < ncols) {
-                    scratch[2 * c + 0] = sV;
-                    scratch[2 * c + 1] = sW;
+                } else if (MULTI && lane == 31 && s >= 62) {  // (its columns: 0 .. ncols - 1)
+                    scratch[c] = make_float4(sV.x, sV.y, sW.x, sW.y);
                 }
             };
             // haplotype boundaries of this task: columns hb(j) = hap_off[hap_begin + j] - col0, hb(n) = ncols
@@ -316,33 +337,48 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
                 const int n_reset = dummies >= 0 ? min(30, dummies / K + 1) : 0;  // lanes with or right below dummy rows
                 for (int j = 0; j <= nh_task; ++j) {
                     const int until = j < nh_task ? (int)(hoff[j] - col0) : nsteps;
-                    // unrolled: the scheduler interleaves one step's I~ chain and shuffles with the following steps' M~
-                    // and D~ (16 measured best of 2-32)
-#pragma unroll 16
-                    for (; s < until; ++s) step(s, Plain{}, 0, 0.f);
+                    while (s < until) {
+                        refill(s);
+                        const int stop = MULTI && strip > 0 ? min(until, (s | 31) + 1) : until;
+                        // unrolled: the scheduler interleaves one step's I~ chain and shuffles with the following steps' M~
+                        // and D~ (16 measured best of 2-32; with the strip boundary 8 of 4, 8 and 16)
+                        constexpr int kUnroll = MULTI ? 8 : 16;
+#pragma unroll kUnroll
+                        for (; s < stop; ++s) step(s, Plain{}, 0, 0.f);
+                    }
                     if (j == nh_task) break;
                     const float init = __ldg(B.hap_init_f + task.hap_begin + j);
                     int l = 0;
 #pragma unroll 1
                     for (; l < n_reset; ++l, s += 2) {
+                        refill(s);
                         step(s, Reset{}, l, init);
+                        refill(s + 1);
                         step(s + 1, Plain{}, 0, 0.f);
                     }
 #pragma unroll 1
                     for (; l < 30; ++l, s += 2) {
+                        refill(s);
                         step(s, Zero{}, l, 0.f);
+                        refill(s + 1);
                         step(s + 1, Plain{}, 0, 0.f);
                     }
+                    refill(s);
                     step(s, Reset{}, 30, init);
+                    refill(s + 1);
                     step(s + 1, Plain{}, 0, 0.f);
                     if (j > 0 && last_strip && lane == 31) emit(task.hap_begin + j - 1);
+                    refill(s + 2);
                     step(s + 2, Reset{}, 31, init);
                     s += 3;
                 }
                 if (last_strip && lane == 31) emit(task.hap_end - 1);
             } else {
 #pragma unroll 2
-                for (; s < nsteps; ++s) step(s, std::integral_constant<int, kCheck>{}, 0, 0.f);
+                for (; s < nsteps; ++s) {
+                    refill(s);
+                    step(s, std::integral_constant<int, kCheck>{}, 0, 0.f);
+                }
             }
             if (MULTI) __syncwarp();
         }
@@ -520,11 +556,13 @@ __global__ void peak_dfma_kernel(double *out, int iters, double x, double y) {
 }
 
 // ---------------------------------------------------------------------------------------------------
-static size_t fp32_smem_bytes(int k, int block) { return (size_t)(block / 32) * ((k + 1) / 2) * kBases * 32 * sizeof(float4); }
+static size_t fp32_smem_bytes(int k, int block, bool multi) {
+    return (size_t)(block / 32) * (((k + 1) / 2) * kBases * 32 + (multi ? 64 : 0)) * sizeof(float4);
+}
 
 template <int K, bool MULTI>
 static int launch_fp32_k(const DevTables &t, const DevBatch &b, int grid, int block, cudaStream_t s) {
-    const size_t smem = fp32_smem_bytes(K, block);
+    const size_t smem = fp32_smem_bytes(K, block, MULTI);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(fp32_bucket_kernel<K, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
@@ -562,9 +600,9 @@ int fp32_kernel_occupancy(int k, int block, int *blocks_per_sm) {
 #define GHMM_OCC(KK)                                                                                              \
     case KK:                                                                                                      \
         e = multi ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fp32_bucket_kernel<KK, true>, block,  \
-                                                                  fp32_smem_bytes(KK, block))                          \
+                                                                  fp32_smem_bytes(KK, block, true))                          \
                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fp32_bucket_kernel<KK, false>, block, \
-                                                                  fp32_smem_bytes(KK, block));                         \
+                                                                  fp32_smem_bytes(KK, block, false));                         \
         break;
         GHMM_OCC(1)
         GHMM_OCC(2)

@@ -91,3 +91,37 @@ def test_short_haplotype_in_a_task_changes_no_other_result():
     assert np.array_equal(out["mixed"][:, :, [1, 2, 3, 5, 6, 7, 8]], out["long"])
     want = oracle.compute_workload(workload.from_pairs([(haps, reads)])).reshape(len(reads), len(haps))
     assert np.abs(out["long"] - want).max() <= 1e-3
+
+
+
+RING_HAPS = (287, 288, 289, 319, 320, 321, 352, 543, 544, 545)
+
+
+@pytest.mark.parametrize("related", [False, True])
+def test_strip_boundaries_around_the_ring(related):
+    """Reads of several strips against haplotypes whose lengths sit around the 32 columns in which a strip's boundary row
+    is read back: one haplotype a task and several, the same bits, and the oracle's values within the FP32 bar.  Unrelated
+    haplotypes: each read fits one, the other pairs go on to FP64; related: leading parts of one sequence, so that most
+    pairs keep their FP32 results."""
+    rng = np.random.default_rng(14)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    haps = [acgt[rng.integers(0, 4, n)] for n in RING_HAPS]
+    if related:
+        haps = [haps[-1][:n] for n in RING_HAPS]
+    reads = []
+    for n in (255, 256, 270, 286, 509, 510, 511, 540):
+        for h in [x for x in haps if len(x) >= n][:3]:
+            o = int(rng.integers(0, len(h) - n + 1))
+            reads.append((h[o:o + n], rng.integers(30, 41, n), np.full(n, 45), np.full(n, 45), np.full(n, 10)))
+    one = workload.from_pairs([(haps, reads)])
+    eng = Engine()
+    try:
+        alone = eng.compute(one)
+        copies = 128
+        with eng.batch(workload.from_pairs([(haps, reads)] * copies)) as b:
+            b.forward(native.MODE_FP32_RERUN)
+            together = b.results().reshape(copies, -1)
+    finally:
+        eng.close()
+    assert np.array_equal(together, np.broadcast_to(alone, together.shape))
+    assert np.abs(alone - oracle.compute_workload(one)).max() <= 1e-3
