@@ -511,7 +511,10 @@ int batch_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s) {
     GHMM_CUDA(b.d_nout.reserve(1), "device output count");
     const size_t s32 = (size_t)b.scratch32_blocks * kWarpsPerBlock * (size_t)b.scratch32_cols * 3;
     GHMM_CUDA(b.d_scratch32.reserve(std::max<size_t>(s32, 1)), "device FP32 strip scratch");
-    const size_t s64 = (size_t)b.fp64_grid * kWarpsPerBlock * (size_t)std::max(b.max_hap_len, 1) * 3;
+    // columns of the FP64 strip scratch per warp: a haplotype, or a run of them (runs end at what fits)
+    const bool runs64 = b.max_hap_len <= kFp64RunCols && b.max_read_len < kFp64SplitRows;
+    const int64_t cols64 = (int64_t)std::max(b.max_hap_len, 1) * (runs64 ? kFp64Run : 1);
+    const size_t s64 = (size_t)b.fp64_grid * kWarpsPerBlock * (size_t)cols64 * 3;
     GHMM_CUDA(b.d_scratch64.reserve(s64), "device FP64 strip scratch");
     GHMM_CUDA(b.d_read_scale.reserve((size_t)std::max<int64_t>(NR, 1)), "device read scales");
 
@@ -557,7 +560,7 @@ int batch_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s) {
     d.scratch32 = b.d_scratch32.p;
     d.scratch32_cols = b.scratch32_cols;
     d.scratch64 = b.d_scratch64.p;
-    d.scratch64_cols = std::max(b.max_hap_len, 1);
+    d.scratch64_cols = cols64;
     d.read_scale = b.d_read_scale.p;
     // the FP32 pass's per-read scale from the uploaded planes (raw batches redo it after their preparation)
     const int e = launch_read_scale(ctx->tables, d, NR, b.d_read_scale.p, ctx->sm_count, s);

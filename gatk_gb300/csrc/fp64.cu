@@ -23,13 +23,16 @@
 //    all lanes once per 16 columns instead of by one lane in every column (two of 22 DP operations a step before).
 //  * Padding is work: a read's rows are split into strips of 32, 64, 96 or 128 rows that cover ceil(R / 32) * 32 rows
 //    instead of whole strips of 128 (reads of 100-250 bases: 191 rows on average instead of 232).
+//  * The wavefront's fill is work too: 31 of some 430 steps of a short read's strip.  A warp therefore takes a run of up to
+//    four neighbouring queue entries of one read and consecutive haplotypes (as routed pairs and double-precision mode
+//    queue them) as one stream of columns, in which each lane resets its state at a haplotype's first column.
 //  * A pair on one warp uses a quarter of one SM.  Jobs are therefore either a pair per warp, its strips one after the
 //    other, or a pair per block: the strips go round the block's four warps, each strip 48 columns behind the one above
 //    it, in lockstep phases of 16 columns.
 // Measured against one pair per warp in strips of 128 rows (one GB300): 537 reads of 800-2,000 bases x haplotypes of
 // 1,500-3,000 (1.6e10 cells) 214 -> 158 ms, 103 of at most 125 GCUPS; 37,978 pairs of 100-250 bases (2.6e9 cells) all in
 // FP64 36.3 -> 27.2 ms; the 5 reruns of a region of 2,000 reads 0.85 -> 0.34 ms; 48 reruns of 260-600 bases x 800
-// 3.6 -> 1.1 ms.
+// 3.6 -> 1.1 ms.  Runs of haplotypes on top: the 37,978 pairs 27.2 -> 26.0 ms.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -58,24 +61,32 @@ struct Unit {
 __device__ __forceinline__ double mul64(double x, double y, Unit u) { return fma(x, y, u.zero); }
 __device__ __forceinline__ double add64(double x, double y, Unit u) { return fma(x, u.one, y); }
 
-// The pair of a job.
+// The read of a job and its haplotypes: n consecutive ones, n > 1 in a warp's runs only.
 struct Pair64 {
-    int64_t roff, out_index;
+    int64_t roff, out_index;  // of the first haplotype's result; the others' follow
     const uint8_t *hb;
-    int read, hap, R, H;
-    int blocks32;  // rows / 32, rounded up: the rows of all strips
-    int pad;       // dummy rows on top of strip 0 (0..31); they hold the row-0 boundary
-    double init, la;
+    int read, hap, n, R, H;   // H: columns of all n haplotypes
+    int blocks32;             // rows / 32, rounded up: the rows of all strips
+    int pad;                  // dummy rows on top of strip 0 (0..31); they hold the row-0 boundary
+    double la;
 };
 
-__device__ __forceinline__ Pair64 load_pair(const DevBatch &B, PairRef pr) {
+// What lanes look up when they start a haplotype, in shared memory per warp: row-0 values and end columns.
+constexpr int kRun64 = kFp64Run;
+struct Run64 {
+    double init[kRun64];
+    int end[kRun64];
+};
+
+__device__ __forceinline__ Pair64 load_pair(const DevBatch &B, PairRef pr, int n = 1) {
     Pair64 P;
     P.read = pr.read;
     P.hap = pr.hap;
+    P.n = n;
     P.roff = B.read_off[pr.read];
     P.R = (int)(B.read_off[pr.read + 1] - P.roff);
     const int64_t hoff = B.hap_off[pr.hap];
-    P.H = (int)(B.hap_off[pr.hap + 1] - hoff);
+    P.H = (int)(B.hap_off[pr.hap + n] - hoff);
     P.hb = B.hap_bases + hoff;
     const int region = B.read_region[pr.read];
     const int64_t nh = B.region_hap_off[region + 1] - B.region_hap_off[region];
@@ -84,7 +95,6 @@ __device__ __forceinline__ Pair64 load_pair(const DevBatch &B, PairRef pr) {
     P.blocks32 = (P.R + 31) / 32;
     P.pad = P.blocks32 * 32 - P.R;
     P.la = 0.0;
-    P.init = 0.0;
     return P;
 }
 
@@ -99,6 +109,8 @@ struct Strip64 {
     uint32_t base[4];
     double gM, gI, gD;     // row above the lane's first row, previous column
     double nxM, nxI, nxD;  // lane 0 below the first strip: the row above at the next column
+    double init;           // row-0 value of the haplotype the lane is in
+    int start, hap;        // first column and ordinal of the haplotype the lane enters next
     int row0, k;           // first row (slot) of the strip, rows per lane
     bool first, last;
 };
@@ -106,12 +118,14 @@ struct Strip64 {
 // Strip `strip` of n strips that share the pair's 32-row blocks as evenly as they go, the larger ones first.
 template <bool RESCALED>
 __device__ __forceinline__ void strip_begin(const DevTables &T, const DevBatch &B, const Pair64 &P, int strip, int n,
-                                            const double *above, Strip64<RESCALED> &S, int lane) {
+                                            double init, const double *above, Strip64<RESCALED> &S, int lane) {
     const int even = P.blocks32 / n, more = P.blocks32 - even * n;
     S.k = even + (strip < more ? 1 : 0);
     S.row0 = 32 * (strip * even + min(strip, more));
     S.first = strip == 0;
     S.last = strip == n - 1;
+    S.start = S.hap = 0;
+    S.init = init;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int p = S.row0 + lane * S.k + k - P.pad;
@@ -157,30 +171,37 @@ __device__ __forceinline__ void strip_begin(const DevTables &T, const DevBatch &
 // Steps [s0, s1) of a strip of K rows per lane: at step s lane l computes column s - l.  The last row of a strip goes
 // to `below` for the next strip; the pair's last row goes to rowM / rowI, 16 steps at a time.
 template <int K, bool RESCALED>
-__device__ __forceinline__ void strip_steps(const Pair64 &P, Strip64<RESCALED> &S, int s0, int s1, const double *above,
-                                            double *below, double *rowM, double *rowI, Unit u, int lane) {
+__device__ __forceinline__ void strip_steps(const Pair64 &P, const Run64 &run, Strip64<RESCALED> &S, int s0, int s1,
+                                            const double *above, double *below, double *rowM, double *rowI, Unit u,
+                                            int lane) {
     for (int s = s0; s < s1; ++s) {
         const int c = s - lane;
         const bool valid = c >= 0 && c < P.H;
         const uint32_t y = valid ? (uint32_t)__ldg(P.hb + c) : 0x200u;
         const bool yn = (y == 'N');
-        if (c == 0) {  // column-0 boundary (lanes compute ahead of their first column)
+        const bool enter = c == S.start;  // a haplotype's column-0 boundary (lanes compute ahead of their first column)
+        if (P.n > 1 && enter) {
+            S.init = run.init[S.hap];
+            S.start = run.end[S.hap];
+            S.hap = min(S.hap + 1, P.n - 1);  // (a lane past the last column resets a state that nothing reads)
+        }
+        double uM = __shfl_up_sync(kFull, S.M[K - 1], 1);  // (the lane below still needs the column before)
+        double uI = __shfl_up_sync(kFull, S.I[K - 1], 1);
+        double uD = __shfl_up_sync(kFull, S.D[K - 1], 1);
+        if (enter) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 S.M[k] = S.I[k] = 0.0;
-                S.D[k] = (S.first && lane * K + k < P.pad) ? P.init : 0.0;
+                S.D[k] = (S.first && lane * K + k < P.pad) ? S.init : 0.0;
             }
             S.gM = S.gI = 0.0;
-            S.gD = (S.first && lane * K - 1 < P.pad) ? P.init : 0.0;
+            S.gD = (S.first && lane * K - 1 < P.pad) ? S.init : 0.0;
         }
-        double uM = __shfl_up_sync(kFull, S.M[K - 1], 1);
-        double uI = __shfl_up_sync(kFull, S.I[K - 1], 1);
-        double uD = __shfl_up_sync(kFull, S.D[K - 1], 1);
         if (lane == 0) {
             if (S.first) {
                 uM = 0.0;
                 uI = 0.0;
-                uD = P.init;
+                uD = S.init;
             } else {
                 uM = S.nxM;
                 uI = S.nxI;
@@ -234,46 +255,34 @@ __device__ __forceinline__ void strip_steps(const Pair64 &P, Strip64<RESCALED> &
     }
 }
 
-// Phase r (steps 16 r .. 16 r + 15) of a strip; the last strip's part of the last row is added to acc, a column per
-// lane.
+// The pair's scale (RESCALED): la = log2 a_R and the initial condition divided by 2^round(la); all lanes.  Fills the
+// warp's table of its haplotypes.
 template <bool RESCALED>
-__device__ __forceinline__ void strip_phase(const Pair64 &P, Strip64<RESCALED> &S, int r, const double *above,
-                                            double *below, double *rowM, double *rowI, double kappa, double &acc,
-                                            Unit u, int lane) {
-    const int s0 = r * kPhase, s1 = min(s0 + kPhase, P.H + 31);
-    switch (S.k) {
-        case 1: strip_steps<1, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
-        case 2: strip_steps<2, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
-        case 3: strip_steps<3, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
-        default: strip_steps<4, RESCALED>(P, S, s0, s1, above, below, rowM, rowI, u, lane); break;
-    }
-    if (S.last) {
-        __syncwarp();
-        const int c = s0 + lane - 31;
-        if (s0 + lane < s1 && c >= 0 && c < P.H)
-            acc += RESCALED ? fma(kappa, rowI[lane], rowM[lane]) : rowM[lane] + rowI[lane];
-        __syncwarp();
-    }
-}
-
-// The pair's scale (RESCALED): la = log2 a_R and the initial condition divided by 2^round(la); all lanes.
-template <bool RESCALED>
-__device__ __forceinline__ void pair_scale(const DevTables &T, const DevBatch &B, Pair64 &P, double &kappa, int lane) {
-    P.init = B.hap_init_d[P.hap];
+__device__ __forceinline__ void pair_scale(const DevTables &T, const DevBatch &B, Pair64 &P, Run64 &run, double &kappa,
+                                           int lane) {
     kappa = 1.0;
-    if (!RESCALED) return;
-    double la = 0.0;
-    for (int p = lane; p < P.R; p += 32) la += __ldg(T.lm2m64 + B.ins[P.roff + p] * 128 + B.dels[P.roff + p]);
+    int shift = 0;
+    if (RESCALED) {
+        double la = 0.0;
+        for (int p = lane; p < P.R; p += 32) la += __ldg(T.lm2m64 + B.ins[P.roff + p] * 128 + B.dels[P.roff + p]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) la += __shfl_xor_sync(kFull, la, o);
-    P.la = la;
-    P.init = scalbn(P.init, -60 - (int)rint(la));
-    const uint8_t ins = B.ins[P.roff + P.R - 1], del = B.dels[P.roff + P.R - 1];
-    kappa = __ldg(T.err_d + ins) / __ldg(T.m2m_d + ins * 128 + del);
+        for (int o = 16; o > 0; o >>= 1) la += __shfl_xor_sync(kFull, la, o);
+        P.la = la;
+        shift = -60 - (int)rint(la);
+        const uint8_t ins = B.ins[P.roff + P.R - 1], del = B.dels[P.roff + P.R - 1];
+        kappa = __ldg(T.err_d + ins) / __ldg(T.m2m_d + ins * 128 + del);
+    }
+    __syncwarp();  // the last job's steps have read the table
+    if (lane < P.n) {
+        run.init[lane] = scalbn(B.hap_init_d[P.hap + lane], shift);
+        run.end[lane] = (int)(B.hap_off[P.hap + lane + 1] - B.hap_off[P.hap]);
+    }
+    __syncwarp();
 }
 
+// The result of haplotype h of the job from the lanes' parts of the sum over its last row.
 template <bool RESCALED>
-__device__ __forceinline__ void pair_emit(const DevBatch &B, const Pair64 &P, double acc, int lane) {
+__device__ __forceinline__ void pair_emit(const DevBatch &B, const Pair64 &P, int h, double acc, int lane) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
     if (lane != 0) return;
@@ -281,23 +290,61 @@ __device__ __forceinline__ void pair_emit(const DevBatch &B, const Pair64 &P, do
         const double rla = rint(P.la);
         const double v = log10(acc) - kLog10Scale64R - (P.la - rla) * 0.30102999566398120;
         if (v >= kRescaledFloor && v <= 0.0) {
-            B.out[P.out_index] = v;
+            B.out[P.out_index + h] = v;
         } else {  // too close to the FP64 range at S' (or not finite): the exact tier recomputes it
             const int idx = atomicAdd(&B.counters[4], 1);
             if ((int64_t)idx < B.rerun_capacity)
-                B.rerun[B.rerun_capacity + idx] = PairRef{P.read, P.hap};
+                B.rerun[B.rerun_capacity + idx] = PairRef{P.read, P.hap + h};
             else
                 atomicExch(&B.counters[3], 1);
         }
     } else {
-        B.out[P.out_index] = log10(acc) - kLog10Scale64;
+        B.out[P.out_index + h] = log10(acc) - kLog10Scale64;
     }
 }
 
-// A pair that needs no wavefront: an empty read or haplotype (-inf, as in Java), or one beyond the strip scratch.
+// What a warp keeps of the sums of a job's last row: the haplotype being summed and this lane's part.
+struct Sum64 {
+    double acc = 0.0;
+    int hap = 0;
+    int end;  // of that haplotype's columns
+};
+
+// Phase r (steps 16 r .. 16 r + 15) of a strip.  After the last strip's, lane l adds the last row's column of step
+// 16 r + l, and the results of the haplotypes that end among these columns are stored.
+template <bool RESCALED>
+__device__ __forceinline__ void strip_phase(const DevBatch &B, const Pair64 &P, const Run64 &run, Strip64<RESCALED> &S, int r,
+                                            const double *above, double *below, double *rowM, double *rowI, double kappa,
+                                            Sum64 &sum, Unit u, int lane) {
+    const int s0 = r * kPhase, s1 = min(s0 + kPhase, P.H + 31);
+    switch (S.k) {
+        case 1: strip_steps<1, RESCALED>(P, run, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+        case 2: strip_steps<2, RESCALED>(P, run, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+        case 3: strip_steps<3, RESCALED>(P, run, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+        default: strip_steps<4, RESCALED>(P, run, S, s0, s1, above, below, rowM, rowI, u, lane); break;
+    }
+    if (!S.last) return;
+    __syncwarp();
+    const int c = s0 + lane - 31;
+    double v = 0.0;
+    if (s0 + lane < s1 && c >= 0) v = RESCALED ? fma(kappa, rowI[lane], rowM[lane]) : rowM[lane] + rowI[lane];
+    __syncwarp();
+    int from = s0 - 31;  // columns [from, s1 - 31) are new
+    while (sum.end <= s1 - 31) {
+        if (c >= from && c < sum.end) sum.acc += v;
+        pair_emit<RESCALED>(B, P, sum.hap, sum.acc, lane);
+        sum.acc = 0.0;
+        from = sum.end;
+        sum.end = ++sum.hap < P.n ? run.end[sum.hap] : INT32_MAX;
+    }
+    if (c >= from && s0 + lane < s1) sum.acc += v;
+}
+
+// A read without bases or a haplotype without columns: -inf, as in Java; one beyond the strip scratch: an error.
 __device__ __forceinline__ bool pair_skipped(const DevBatch &B, const Pair64 &P, bool writer) {
     if (P.R == 0 || P.H == 0) {
-        if (writer) B.out[P.out_index] = -INFINITY;
+        if (writer)
+            for (int h = 0; h < P.n; ++h) B.out[P.out_index + h] = -INFINITY;
         return true;
     }
     if (P.H > B.scratch64_cols && P.blocks32 > 1) {
@@ -316,6 +363,7 @@ template <bool RESCALED>
 __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables T, DevBatch B, bool long_reads,
                                                                       Unit u) {
     __shared__ double row_sum[kWarps64][2][kPhase];
+    __shared__ Run64 runs[kWarps64];
     __shared__ int job;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const PairRef *queue = RESCALED ? B.rerun : B.rerun + B.rerun_capacity;
@@ -324,23 +372,51 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
     double *const block_scratch = B.scratch64 + (int64_t)blockIdx.x * kWarps64 * B.scratch64_cols * 3;
     double *const mine = block_scratch + (int64_t)warp * B.scratch64_cols * 3;
     double *const rowM = row_sum[warp][0], *const rowI = row_sum[warp][1];
+    Run64 &run = runs[warp];
     Strip64<RESCALED> S;
     double kappa;
-    if (total > (int)gridDim.x * kWarps64 && !long_reads) {
-        for (bool first = true;;) {
-            const int t = draw_entry(cursor, first, lane);
-            if (t >= total) break;
-            Pair64 P = load_pair(B, queue[t]);
-            if (pair_skipped(B, P, lane == 0)) continue;
-            pair_scale<RESCALED>(T, B, P, kappa, lane);
-            const int n = (P.blocks32 + 3) / 4, phases = (P.H + 31 + kPhase - 1) / kPhase;
-            double acc = 0.0;
-            for (int strip = 0; strip < n; ++strip) {
-                __syncwarp();  // the strip above has written its last row
-                strip_begin<RESCALED>(T, B, P, strip, n, mine, S, lane);
-                for (int r = 0; r < phases; ++r) strip_phase<RESCALED>(P, S, r, mine, mine, rowM, rowI, kappa, acc, u, lane);
+    const int warps = (int)gridDim.x * kWarps64;
+    if (total > warps && !long_reads) {
+        // entries drawn several at a time while many a warp are left, one by one towards the end
+        for (;;) {
+            int t0 = 0, draw = 1;
+            if (lane == 0) {
+                const int left = total - *reinterpret_cast<volatile int *>(cursor);
+                draw = max(1, min(kRun64, left / (2 * warps)));
+                t0 = atomicAdd(cursor, draw);
             }
-            pair_emit<RESCALED>(B, P, acc, lane);
+            t0 = __shfl_sync(kFull, t0, 0);
+            draw = __shfl_sync(kFull, draw, 0);
+            if (t0 >= total) break;
+            const int t1 = min(t0 + draw, total);
+            for (int t = t0; t < t1;) {
+                const PairRef pr = queue[t];
+                // a run: the same read, the haplotype after the last one's, no empty ones, within the strip scratch
+                int n = 1;
+                const int64_t h0 = B.hap_off[pr.hap];
+                int64_t end = B.hap_off[pr.hap + 1];
+                while (t + n < t1 && end > h0) {
+                    const PairRef next = queue[t + n];
+                    if (next.read != pr.read || next.hap != pr.hap + n) break;
+                    const int64_t e = B.hap_off[next.hap + 1];
+                    if (e == end || e - h0 > B.scratch64_cols) break;
+                    end = e;
+                    ++n;
+                }
+                t += n;
+                Pair64 P = load_pair(B, pr, n);
+                if (pair_skipped(B, P, lane == 0)) continue;
+                pair_scale<RESCALED>(T, B, P, run, kappa, lane);
+                const int strips = (P.blocks32 + 3) / 4, phases = (P.H + 31 + kPhase - 1) / kPhase;
+                Sum64 sum;
+                sum.end = run.end[0];
+                for (int strip = 0; strip < strips; ++strip) {
+                    __syncwarp();  // the strip above has written its last row
+                    strip_begin<RESCALED>(T, B, P, strip, strips, run.init[0], mine, S, lane);
+                    for (int r = 0; r < phases; ++r)
+                        strip_phase<RESCALED>(B, P, run, S, r, mine, mine, rowM, rowI, kappa, sum, u, lane);
+                }
+            }
         }
         return;
     }
@@ -357,7 +433,7 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
         if (t >= total) break;
         Pair64 P = load_pair(B, queue[t]);
         if (pair_skipped(B, P, threadIdx.x == 0)) continue;
-        pair_scale<RESCALED>(T, B, P, kappa, lane);
+        pair_scale<RESCALED>(T, B, P, run, kappa, lane);
         // strips of at most 128 rows, a multiple of four of them where the rows allow; strip s runs on warp s % 4 from
         // phase start(s) = (s / 4) round + (s % 4) lag on, round being a strip's phases and long enough for the strip
         // that wraps round to warp 0 to stay behind the one above it on warp 3
@@ -366,11 +442,12 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
         const int round = max(phases, kStripLag * kWarps64);
         const int end = (n - 1) / kWarps64 * round + (n - 1) % kWarps64 * kStripLag + phases;
         int strip = warp, start = warp * kStripLag;
-        double acc = 0.0;
+        Sum64 sum;
+        sum.end = P.H;
         for (int p = 0; p < end; ++p) {
             if (strip < n && p >= start) {
-                if (p == start) strip_begin<RESCALED>(T, B, P, strip, n, above, S, lane);
-                strip_phase<RESCALED>(P, S, p - start, above, mine, rowM, rowI, kappa, acc, u, lane);
+                if (p == start) strip_begin<RESCALED>(T, B, P, strip, n, run.init[0], above, S, lane);
+                strip_phase<RESCALED>(B, P, run, S, p - start, above, mine, rowM, rowI, kappa, sum, u, lane);
                 if (p - start == phases - 1) {
                     strip += kWarps64;
                     start += round;
@@ -378,7 +455,6 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
             }
             __syncthreads();
         }
-        if (warp == (n - 1) % kWarps64) pair_emit<RESCALED>(B, P, acc, lane);
     }
 }
 

@@ -49,6 +49,22 @@ def test_fp64_strip_shapes(case):
     assert np.max(np.abs(got[differ] - want[differ]), initial=0.0) <= 1e-9
 
 
+def test_fp64_runs_of_haplotypes():
+    """Enough pairs for a warp to take runs of a read's haplotypes as one stream: short, empty and ordinary haplotypes
+    following one another, results ending several to a phase of 16 columns.  |d| <= 1e-9 as above."""
+    rng = np.random.default_rng(15)
+    haps = [1, 2, 15, 16, 17, 0, 31, 32, 33, 3, 3, 3, 3, 48, 97, 210, 0, 0, 130]
+    wl = workload.from_pairs([_region(rng, EDGES, haps) for _ in range(60)])  # 23,940 pairs
+    eng = Engine(use_double_precision=True)
+    try:
+        got = eng.compute(wl)
+    finally:
+        eng.close()
+    want = oracle.compute_workload(wl)
+    differ = got != want  # (infinities are equal)
+    assert np.max(np.abs(got[differ] - want[differ]), initial=0.0) <= 1e-9
+
+
 def test_results_do_not_depend_on_the_task_split():
     """Regions called one by one (cut down to a haplotype a task) and in one batch of many (whole regions a task) give
     the same bits, several strips included."""
