@@ -75,11 +75,13 @@ int queue_launch(ghmm_queue *q, int i, QueueUnit &u) {
         rc = raw_prepare_device(ctx, b, u.mapq.data(), u.max_len, &q->prep, q->stream[i]);
         if (rc) return rc;
     }
-    if (q->serial_fp32) {  // the FP32 pass after the other slot's (its FP64 reruns and copies still overlap)
-        const int o = 1 - i;
-        if (q->inflight[o] && q->slot[o].events_ready)
-            GHMM_CUDA(cudaStreamWaitEvent(q->stream[i], q->slot[o].ev[2], 0), "wait for the previous FP32 pass");
-    }
+    // The FP32 pass after the other slot's (its FP64 reruns and copies still overlap): two batches' bucket kernels side
+    // by side ran slower than in turn, or as fast (workload 0 in one call: 5,000 regions 40.8 against 34.9 ms, 1,200
+    // 10.3 and 9.15, 600 the same; workload 1 the same from 200 to 6,000 regions; the streaming queue over 30,000
+    // regions of workload 4 in batches of 2e11 cells: 3,698 against 3,848 GCUPS).
+    const int o = 1 - i;
+    if (q->inflight[o] && q->slot[o].events_ready)
+        GHMM_CUDA(cudaStreamWaitEvent(q->stream[i], q->slot[o].ev[2], 0), "wait for the previous FP32 pass");
     rc = batch_enqueue(ctx, b, q->mode, q->stream[i]);
     if (rc) return rc;
     if (b.n_out > 0) {
@@ -148,9 +150,9 @@ void queue_worker(ghmm_queue *q) {
                     if (q->inflight[i] && (oldest < 0 || q->inflight_seq[i] < q->inflight_seq[oldest])) oldest = i;
                 if (oldest >= 0) {
                     // nothing to marshal: retire the oldest batch once it is done, polling so that a newly
-                    // sealed batch is taken up while it runs
+                    // sealed batch is taken up while it runs (a pipelined call ends with the last of these polls)
                     if (cudaEventQuery(q->slot[oldest].ev[4]) != cudaErrorNotReady) break;
-                    q->cv_work.wait_for(lk, std::chrono::microseconds(200));
+                    q->cv_work.wait_for(lk, std::chrono::microseconds(20));
                     oldest = -1;
                     continue;
                 }
@@ -233,9 +235,6 @@ int queue_open(ghmm_ctx *ctx, int64_t batch_cells, ghmm_queue **out, const ghmm_
     auto *q = new ghmm_queue();
     q->ctx = ctx;
     q->batch_cells = batch_cells > 0 ? batch_cells : (int64_t)2e11;
-    // a streaming queue's batches run their FP32 passes in turn (workload 4 through the queue, 30,000 regions in
-    // batches of 2e11 cells: 3,848 against 3,698 GCUPS side by side)
-    q->serial_fp32 = true;
     q->mode = ctx->double_precision ? GHMM_MODE_FP64 : GHMM_MODE_FP32_RERUN;
     if (raw_prep) queue_set_raw(q, raw_prep, bound);
     for (auto &st : q->stream) {
@@ -300,35 +299,28 @@ std::unique_ptr<QueueUnit> borrowed_unit(const Source &src, int64_t g0, int64_t 
 }
 
 
-// Raw reads (mapq non-NULL, src.regions over the raw view's reads): every batch gets the read preparation prep on
-// the device after its upload.
-// Region cuts [0 = c_0 < c_1 < ... = G] of a pipelined call over regions of the given cells.  Below 5e11 cells: three
-// chunks, after 1/8 and 1/2 of the cells, because each chunk's launches, graph capture and kernel tails cost a fixed
-// time (workload 1 end to end through ghmm_compute_regions: 95.6 ms against 101.5 ms for the finer cut at 3,000
-// regions; the regular calls run below 1.5e11 cells as one batch, the one-shot PD-HMM calls in chunks down to 8
-// regions, which gain or lose nothing measurable against one chunk at 1,000 regions).  Above: 1/16 of the cells first, each next chunk 2.5 times the last up to
-// 1/3, so the first marshal the device waits for stays short (281.5 ms against 285.8 ms for three chunks at 10,000
-// regions).  No cut leaves fewer than 8 regions behind it.
-std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells) {
+// A call runs as a pipeline from 250,000 pairs on, where its marshal, upload and results, which go with the pairs and
+// their bytes, cost more than what the extra batches' launches and kernel tails do.  End to end, one batch against the
+// pipeline: workload 0 at 400 regions (205,000 pairs) 4.58 and 4.55 ms, at 600 6.60 and 5.74, at 5,000 56.8 and 34.8;
+// workload 1 at 150 regions (200,000 pairs) 5.84 and 5.85 ms, at 300 10.3 and 9.7, at 1,000 34.6 and 29.2; workload 3
+// at 40,000 regions (320,000 pairs) 26.1 and 22.0.  Of few long pairs only inputs of 1.5e11 cells are cut, which bounds
+// a batch's memory: workload 2 at 100 regions (35,000 pairs, 1.1e11 cells) takes 1,011 and 1,024 ms.
+bool pipelines(int64_t cells, int64_t pairs, int64_t regions) {
+    return regions >= 4 && (pairs >= kPipelineMinPairs || cells >= kPipelineMinCells);
+}
+
+// Region cuts [0 = c_0 < c_1 < ... = G] of a pipelined call over regions of the given cells: a small chunk first, each
+// next one 2.5 times the last up to 1/3 of the cells, so the first marshal the device waits for stays short.  The
+// first chunk is 1/8 of the cells below 1e11 and 1/16 above, where an eighth is long enough to wait for (end to end
+// with 1/8 and 1/16: workload 0 at 1,200 regions, 2.8e10 cells, 9.1 and 9.7 ms, at 5,000, 1.15e11, 34.8 and 34.0;
+// workload 1 at 400 regions, 4e10, 12.2 and 12.7, at 3,000, 3.2e11, 81.6 and 80.1, at 6,000 162.2 and 158.2).  No cut
+// leaves fewer than 8 regions behind it.
+std::vector<int64_t> growing_cuts(const std::vector<int64_t> &cells) {
     const int64_t G = (int64_t)cells.size();
     int64_t total = 0;
     for (int64_t c : cells) total += c;
     std::vector<int64_t> cut{0};
-    if (total < kPipelineLargeCells) {
-        const int64_t marks[2] = {total / 8, total / 2};
-        int64_t c = 0;
-        int m = 0;
-        for (int64_t g = 0; g < G && m < 2; g++) {
-            c += cells[(size_t)g];
-            if (c >= marks[m] && G - g - 1 >= 8) {
-                cut.push_back(g + 1);
-                m++;
-            }
-        }
-        cut.push_back(G);
-        return cut;
-    }
-    int64_t target = std::max<int64_t>(total / 16, 1);
+    int64_t target = std::max<int64_t>(total / (total < (int64_t)1e11 ? 8 : 16), 1);
     for (int64_t g0 = 0; g0 < G;) {
         int64_t g1 = g0, c = 0;
         while (g1 < G && (c < target || g1 == g0)) c += cells[(size_t)g1++];
@@ -340,6 +332,31 @@ std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells) {
     return cut;
 }
 
+// Region cuts of a one-shot PD-HMM call.  Below 5e11 cells: three chunks, after 1/8 and 1/2 of the cells, because each
+// chunk's launches, graph capture and kernel tails cost a fixed time.  Above: growing_cuts.  No cut leaves fewer than
+// 8 regions behind it.
+std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells) {
+    const int64_t G = (int64_t)cells.size();
+    int64_t total = 0;
+    for (int64_t c : cells) total += c;
+    if (total >= kPipelineLargeCells) return growing_cuts(cells);
+    std::vector<int64_t> cut{0};
+    const int64_t marks[2] = {total / 8, total / 2};
+    int64_t c = 0;
+    int m = 0;
+    for (int64_t g = 0; g < G && m < 2; g++) {
+        c += cells[(size_t)g];
+        if (c >= marks[m] && G - g - 1 >= 8) {
+            cut.push_back(g + 1);
+            m++;
+        }
+    }
+    cut.push_back(G);
+    return cut;
+}
+
+// Raw reads (mapq non-NULL, src.regions over the raw view's reads): every batch gets the read preparation prep on
+// the device after its upload.
 int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_t> &reg_cells,
                       const std::vector<int64_t> &reg_out, double *out, const int32_t *mapq,
                       int32_t max_len, const ghmm_read_prep *prep, const RouteBound *bound) {
@@ -354,12 +371,6 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
         q->error_msg.clear();
         q->mode = ctx->double_precision ? GHMM_MODE_FP64 : GHMM_MODE_FP32_RERUN;
         queue_set_raw(q, mapq ? prep : nullptr, bound);
-        // the large schedule's chunks run their FP32 passes in turn: bucket kernels of two such chunks side by side
-        // ran slower than one after the other (workload 1 end to end at 10,000 regions: 290 against 282 ms), while the
-        // small schedule's chunks gain from filling each other's kernel tails (42.4 against 44.5 ms at 1,000 regions)
-        int64_t total = 0;
-        for (int64_t c : reg_cells) total += c;
-        q->serial_fp32 = total >= kPipelineLargeCells;
     }
     const int64_t G = src.n_regions;
     std::vector<int64_t> first_read;  // raw reads: the batch's reads' mapping qualities go with the batch
@@ -367,7 +378,7 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
         first_read.assign((size_t)G + 1, 0);
         for (int64_t g = 0; g < G; g++) first_read[(size_t)g + 1] = first_read[(size_t)g] + src.regions[g].n_reads;
     }
-    const std::vector<int64_t> cut = pipeline_cuts(reg_cells);
+    const std::vector<int64_t> cut = growing_cuts(reg_cells);
     for (size_t i = 0; i + 1 < cut.size(); i++) {
         const int64_t g0 = cut[i], g1 = cut[i + 1];
         int64_t c = 0;
@@ -434,7 +445,7 @@ int compute_sync(ghmm_ctx *ctx, const Source &src, double *out) {
     int64_t total = 0;
     for (auto c : cells) total += c;
     if (outo.back() > 0 && !out) return fail(ctx, GHMM_ERR_ARG, "NULL output");
-    if (total >= kPipelineMinCells && src.n_regions >= 4) return pipelined_compute(ctx, src, cells, outo, out);
+    if (pipelines(total, outo.back(), src.n_regions)) return pipelined_compute(ctx, src, cells, outo, out);
     ghmm_batch &b = ctx->scratch_batch;
     int rc = batch_marshal(ctx, src, b);
     if (!rc) rc = batch_upload(ctx, b, ctx->stream);

@@ -253,7 +253,7 @@ int ghmm_compute_regions_raw(ghmm_ctx *ctx, const ghmm_raw_region *regions, int3
         int64_t total = 0;
         for (auto c : cells) total += c;
         if (outo.back() > 0 && !out) return fail(ctx, GHMM_ERR_ARG, "NULL output");
-        if (total >= kPipelineMinCells && n_regions >= 4)
+        if (pipelines(total, outo.back(), n_regions))
             return pipelined_compute(ctx, src, cells, outo, out, v.mapq.data(), v.max_len, prep,
                                      v.has_bound ? &v.bound : nullptr);
     }

@@ -296,8 +296,6 @@ struct ghmm_queue {
     std::vector<double> str_tables;
     bool has_bound = false;
     RouteBound bound;
-    // each batch's kernels wait for the FP32 pass of the batch in the other slot (streaming queues, large pipelined calls)
-    bool serial_fp32 = false;
     // worker-owned
     ghmm_batch slot[2];
     cudaStream_t stream[2]{};
@@ -344,10 +342,10 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s);
 int pd_forward_finish(ghmm_ctx *ctx, ghmm_batch &b);
 
 // queue.cpp.  Large synchronous inputs run as a pipeline of batches through the context's own queue: the first
-// batch is small so that the GPU starts early, later ones grow to a third of the input.  Below 1.5e11 cells one batch
-// is faster, the marshal being shorter than what the extra batches' launches and kernel tails cost (workload 1 end to
-// end at 1,000 regions, 1.09e11 cells: 38.7 ms in one batch against 42.4 ms in three).
+// batch is small so that the GPU starts early, later ones grow to a third of the input.
 constexpr int64_t kPipelineMinCells = (int64_t)1.5e11;
+constexpr int64_t kPipelineMinPairs = 250000;
+bool pipelines(int64_t cells, int64_t pairs, int64_t regions);  // whether a synchronous call of that size is cut
 int queue_open(ghmm_ctx *ctx, int64_t batch_cells, ghmm_queue **out, const ghmm_read_prep *raw_prep = nullptr,
                const RouteBound *bound = nullptr);
 void queue_close(ghmm_queue *q);
@@ -361,9 +359,10 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
                       int32_t max_len = 0, const ghmm_read_prep *prep = nullptr, const RouteBound *bound = nullptr);
 bool region_sizes(const Source &src, std::vector<int64_t> &cells, std::vector<int64_t> &outo, int threads);
 int compute_sync(ghmm_ctx *ctx, const Source &src, double *out);
-// cells from which a pipelined call takes the large schedule (growing chunks, FP32 passes in turn)
+// cells from which one-shot PD-HMM calls take growing chunks
 constexpr int64_t kPipelineLargeCells = (int64_t)5e11;
-std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells);  // region cuts of a pipelined call
+std::vector<int64_t> growing_cuts(const std::vector<int64_t> &cells);   // region cuts of a pipelined call
+std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells);  // region cuts of a one-shot PD-HMM call
 
 // pd_host.cpp
 int pd_marshal(ghmm_ctx *ctx, const ghmm_pd_region *regs, int64_t G, ghmm_batch &b, const RouteBound *bound);

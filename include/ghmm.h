@@ -185,8 +185,8 @@ int ghmm_done(ghmm_ctx *ctx);
 int ghmm_last_error(const ghmm_ctx *ctx, char *buf, size_t buf_len);
 
 /* Batcher: many regions in one call (regions of HaplotypeCallerEngine.callRegion batched together).
- * out receives each region's read-major block back to back, in region order.  Inputs of 1.5e11 cells or
- * more run as a pipeline of batches (the first small, later ones up to a third of the input) on the
+ * out receives each region's read-major block back to back, in region order.  Inputs of 250,000 pairs or
+ * 1.5e11 cells run as a pipeline of batches (the first small, later ones up to a third of the input) on the
  * context's internal queue, so that marshalling overlaps the kernels; the results are the same. */
 int ghmm_compute_regions(ghmm_ctx *ctx, const ghmm_region *regions, int32_t n_regions, double *out);
 
@@ -402,8 +402,7 @@ int ghmm_debug_tables(ghmm_ctx *ctx, double *err, double *prob, double *m2m);
  * the general PD kernel, GHMM_ERR_ARG for bad arguments. */
 int ghmm_debug_pd_ops(const uint8_t *bases, const uint8_t *pd_flags, int32_t H, uint8_t *ops, uint8_t *codes);
 
-/* Debug/test (no device needed): the chunks a pipelined call cuts regions of these cells into (ghmm_compute_regions,
- * _flat and _raw on inputs of 1.5e11 cells or more; the one-shot PD-HMM calls on every input): cuts[0] = 0 <
+/* Debug/test (no device needed): the chunks a one-shot PD-HMM call cuts regions of these cells into: cuts[0] = 0 <
  * cuts[1] < ... = n_regions, chunk i being regions [cuts[i], cuts[i + 1]).  Below 5e11 cells the cuts fall where
  * the running sum of cells first reaches 1/8 and 1/2 of the total; from 5e11, the first chunk takes 1/16 of the cells
  * and each next one 2.5 times the last, up to 1/3.  No cut leaves fewer than 8 regions behind it.  Writes
