@@ -368,15 +368,20 @@ int pd_forward_finish(ghmm_ctx *ctx, ghmm_batch &b) {
 
 // The one-shot PD-HMM calls in chunks of regions, pipelined on two streams: chunk i+1 is marshalled on the host and
 // enqueued (upload, preparation, forward) on the other slot's stream while chunk i runs, so its kernels start as
-// chunk i's last tasks leave SMs free; then chunk i's results are read.  Chunks as pipeline_cuts cuts them (below
-// 5e11 cells three, of 1/8, 3/8 and 1/2 of the cells: on 1,000 regions of workload 1 with PD flags, 85 ms a call
-// against 112 ms for the finer cut of large inputs and 84 ms unchunked; on 3,000 regions, 198 ms against 209 ms and
-// 232 ms).  host(g0, g1, slot) stages regions [g0, g1) in ctx->pd_batch[slot]; device(slot, stream) uploads it (and
-// prepares raw reads).
+// chunk i's last tasks leave SMs free; then chunk i's results are read.  Below 1.5e10 cells one chunk: two more uploads,
+// graphs, kernel tails and waits cost more than what the overlap hides (regions of workload 1 with PD flags, one chunk
+// and three: 14 regions 1.27 and 1.51 ms, 20 2.83 and 3.43, 70 5.87 and 6.55, 140 at 1.2e10 cells 9.1 and 9.7, but 40
+// 3.8 and 3.4; 200 at 1.8e10 12.5 and 11.2, 300 18.7 and 16.4, 600 36.0 and 31.4).  Above, chunks as pipeline_cuts
+// cuts them (below 5e11 cells three, of 1/8, 3/8 and 1/2 of the cells, where the growing cuts of regular calls took
+// 12.1, 19.3 and 34.7 ms at 200, 300 and 600 regions).  host(g0, g1, slot) stages regions [g0, g1) in
+// ctx->pd_batch[slot]; device(slot, stream) uploads it (and prepares raw reads).
 int pd_pipelined(ghmm_ctx *ctx, const std::vector<int64_t> &cells, const std::vector<int64_t> &outo, double *out,
                  const std::function<int(int64_t, int64_t, int)> &host,
                  const std::function<int(int, cudaStream_t)> &device) {
-    const std::vector<int64_t> cut = pipeline_cuts(cells);
+    int64_t total = 0;
+    for (int64_t c : cells) total += c;
+    const std::vector<int64_t> cut = total < kPdPipelineMinCells ? std::vector<int64_t>{0, (int64_t)cells.size()}
+                                                                 : pipeline_cuts(cells);
     if (!ctx->pd_stream2)
         GHMM_CUDA(cudaStreamCreateWithFlags(&ctx->pd_stream2, cudaStreamNonBlocking), "cudaStreamCreate");
     const cudaStream_t streams[2] = {ctx->stream, ctx->pd_stream2};
