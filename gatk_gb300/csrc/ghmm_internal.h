@@ -133,10 +133,12 @@ constexpr uint32_t kPdOpSnpAllBut = 128;  // with kPdOpSnp: three bases match, b
 int launch_pd_bucket(const DevTables &t, const DevBatch &b, const PdPlanes &pd, int key, int grid, cudaStream_t s);
 int pd_bucket_occupancy(int key, int *blocks_per_sm);
 int pd_kernel_occupancy(int *blocks_per_sm);
-// PD pairs [begin, begin + count) of the pair list (count_dev: the count in device memory), K rows per lane, in
-// FP32 (underflows queued for FP64 at rerun[rerun_capacity..)) or FP64; cursor is the counter the warps draw from.
+// PD pairs [begin, begin + count) of the pair list, K rows per lane, in FP32 (underflows queued for FP64 at
+// rerun[rerun_capacity..)) or FP64; cursor is the counter the warps draw from.
 int launch_pd(const DevTables &t, const DevBatch &b, const PdPlanes &p, int k, bool fp32, int begin, int count,
-              int cursor, const int32_t *count_dev, int grid, cudaStream_t s);
+              int cursor, int grid, cudaStream_t s);
+// The queued PD pairs (counters[kCounterPdRerun] of them) in FP64.
+int launch_pd_rerun(const DevTables &t, const DevBatch &b, const PdPlanes &p, int grid, cudaStream_t s);
 constexpr int kPdMaxK = 4;          // PD kernel: rows per lane 1..4 in FP64
 constexpr int kPdMaxK32 = 8;        // and 1..8 in FP32
 constexpr int kCounterPdBase = 40;  // counters[40 + K]: PD FP64 task cursors (inside the 64 counters, above the buckets)

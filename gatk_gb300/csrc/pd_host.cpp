@@ -324,14 +324,13 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s) 
     for (int kk = maxk; kk >= 1; --kk) {  // longest strips first
         if (kcount[kk] == 0) continue;
         const int cursor = (fp32 ? kCounterPdF32Base : kCounterPdBase) + kk;
-        int e = launch_pd(ctx->tables, b.dev, b.pd, kk, fp32, (int)kbegin[kk], (int)kcount[kk], cursor, nullptr, grid, s);
+        int e = launch_pd(ctx->tables, b.dev, b.pd, kk, fp32, (int)kbegin[kk], (int)kcount[kk], cursor, grid, s);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "PD-HMM launch");
         launches++;
     }
     GHMM_CUDA(cudaEventRecord(b.ev[4], s), "event");
     if (fp32) {  // the FP32 pass's underflows, queued at rerun[capacity..), in FP64
-        int e = launch_pd(ctx->tables, b.dev, b.pd, kPdMaxK, false, (int)b.dev.rerun_capacity, 0,
-                          kCounterPdRerunCursor, b.d_counters.p + kCounterPdRerun, grid, s);
+        int e = launch_pd_rerun(ctx->tables, b.dev, b.pd, grid, s);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "PD-HMM FP64 rerun launch");
         launches++;
     }
@@ -368,13 +367,12 @@ int pd_forward_finish(ghmm_ctx *ctx, ghmm_batch &b) {
 
 // The one-shot PD-HMM calls in chunks of regions, pipelined on two streams: chunk i+1 is marshalled on the host and
 // enqueued (upload, preparation, forward) on the other slot's stream while chunk i runs, so its kernels start as
-// chunk i's last tasks leave SMs free; then chunk i's results are read.  Below 1.5e10 cells one chunk: two more uploads,
+// chunk i's last tasks leave SMs free; then chunk i's results are read.  Below 2e9 cells one chunk: two more uploads,
 // graphs, kernel tails and waits cost more than what the overlap hides (regions of workload 1 with PD flags, one chunk
-// and three: 14 regions 1.27 and 1.51 ms, 20 2.83 and 3.43, 70 5.87 and 6.55, 140 at 1.2e10 cells 9.1 and 9.7, but 40
-// 3.8 and 3.4; 200 at 1.8e10 12.5 and 11.2, 300 18.7 and 16.4, 600 36.0 and 31.4).  Above, chunks as pipeline_cuts
-// cuts them (below 5e11 cells three, of 1/8, 3/8 and 1/2 of the cells, where the growing cuts of regular calls took
-// 12.1, 19.3 and 34.7 ms at 200, 300 and 600 regions).  host(g0, g1, slot) stages regions [g0, g1) in
-// ctx->pd_batch[slot]; device(slot, stream) uploads it (and prepares raw reads).
+// and three: 14 regions 1.26 and 1.50 ms, 20 at 1.1e9 cells 2.00 and 2.55; 40 at 2.6e9 2.92 and 2.75, 100 6.6 and 6.2,
+// 300 17.8 and 15.0).  Above, chunks as pipeline_cuts cuts them (below 5e11 cells three, of 1/8, 3/8 and 1/2 of the
+// cells, which were 7 to 15 % faster than the growing cuts of regular calls from 200 to 600 regions).  host(g0, g1, slot)
+// stages regions [g0, g1) in ctx->pd_batch[slot]; device(slot, stream) uploads it (and prepares raw reads).
 int pd_pipelined(ghmm_ctx *ctx, const std::vector<int64_t> &cells, const std::vector<int64_t> &outo, double *out,
                  const std::function<int(int64_t, int64_t, int)> &host,
                  const std::function<int(int, cudaStream_t)> &device) {

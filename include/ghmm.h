@@ -402,7 +402,7 @@ int ghmm_debug_tables(ghmm_ctx *ctx, double *err, double *prob, double *m2m);
  * the general PD kernel, GHMM_ERR_ARG for bad arguments. */
 int ghmm_debug_pd_ops(const uint8_t *bases, const uint8_t *pd_flags, int32_t H, uint8_t *ops, uint8_t *codes);
 
-/* Debug/test (no device needed): the chunks a one-shot PD-HMM call of 1.5e10 cells or more cuts regions of these
+/* Debug/test (no device needed): the chunks a one-shot PD-HMM call of 2e9 cells or more cuts regions of these
  * cells into (below, it runs as one): cuts[0] = 0 < cuts[1] < ... = n_regions, chunk i being regions
  * [cuts[i], cuts[i + 1]).  Below 5e11 cells the cuts fall where the running sum of cells first reaches 1/8 and 1/2 of
  * the total; from 5e11, the first chunk takes 1/16 of the cells and each next one 2.5 times the last, up to 1/3.  No
