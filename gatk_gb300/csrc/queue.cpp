@@ -200,6 +200,12 @@ void queue_submit(ghmm_queue *q, std::unique_ptr<QueueUnit> u) {
     q->cv_work.notify_all();
 }
 
+// Hand the open unit over as a full batch; the next one may be twice as large, up to the queue's batch size.
+void queue_seal(ghmm_queue *q) {
+    queue_submit(q, std::move(q->open));
+    q->next_cells = std::min(2 * q->next_cells, q->batch_cells);
+}
+
 int queue_wait_all(ghmm_queue *q) {
     std::unique_lock<std::mutex> lk(q->mu);
     q->cv_done.wait(lk, [&] { return q->retired == q->submitted; });
@@ -235,6 +241,8 @@ int queue_open(ghmm_ctx *ctx, int64_t batch_cells, ghmm_queue **out, const ghmm_
     auto *q = new ghmm_queue();
     q->ctx = ctx;
     q->batch_cells = batch_cells > 0 ? batch_cells : (int64_t)2e11;
+    q->first_cells = batch_cells > 0 ? batch_cells : kQueueFirstCells;
+    q->next_cells = q->first_cells;
     q->mode = ctx->double_precision ? GHMM_MODE_FP64 : GHMM_MODE_FP32_RERUN;
     if (raw_prep) queue_set_raw(q, raw_prep, bound);
     for (auto &st : q->stream) {
@@ -565,7 +573,7 @@ int ghmm_queue_push_raw(ghmm_queue *q, const ghmm_raw_region *regions, int32_t n
         q->info.n_regions += n_regions;
         q->info.n_pairs += n_out;
     }
-    if (u.cells >= q->batch_cells) queue_submit(q, std::move(q->open));
+    if (u.cells >= q->next_cells) queue_seal(q);
     return queue_status(q);
 }
 
@@ -638,7 +646,7 @@ int ghmm_queue_push(ghmm_queue *q, const ghmm_region *regions, int32_t n_regions
         q->info.n_regions += n_regions;
         q->info.n_pairs += n_out;
     }
-    if (u.cells >= q->batch_cells) queue_submit(q, std::move(q->open));
+    if (u.cells >= q->next_cells) queue_seal(q);
     return queue_status(q);
 }
 
@@ -646,6 +654,7 @@ int ghmm_queue_flush(ghmm_queue *q) {
     if (!q) return GHMM_ERR_STATE;
     if (q->open && q->open->n_regions > 0) queue_submit(q, std::move(q->open));
     q->open.reset();
+    q->next_cells = q->first_cells;
     queue_wait_all(q);
     return queue_status(q);
 }

@@ -228,7 +228,7 @@ struct ghmm_ctx {
 
 // -------------------------------------------------------------------------------------------------
 // Streaming queue: regions are pushed as they arrive and gathered into batches of about batch_cells
-// cells; a worker thread marshals each full batch into one of two slots (pinned + device buffers, one
+// cells (by default growing ones, kQueueFirstCells); a worker thread marshals each full batch into one of two slots (pinned + device buffers, one
 // CUDA stream each) and launches it, so the marshal of batch k+1 on the host, the upload of batch k+1
 // and the kernels of batch k overlap, and the two streams fill each other's kernel tails.
 
@@ -278,6 +278,7 @@ struct QueueUnit {
 struct ghmm_queue {
     ghmm_ctx *ctx = nullptr;
     int64_t batch_cells = 0;
+    int64_t first_cells = 0, next_cells = 0;  // cells at which the first, the open unit is full
     int mode = GHMM_MODE_FP32_RERUN;
     std::unique_ptr<QueueUnit> open;  // filled by push on the caller's thread
     std::mutex mu;
@@ -346,6 +347,13 @@ int pd_forward_finish(ghmm_ctx *ctx, ghmm_batch &b);
 constexpr int64_t kPipelineMinCells = (int64_t)1.5e11;
 constexpr int64_t kPipelineMinPairs = 250000;
 bool pipelines(int64_t cells, int64_t pairs, int64_t regions);  // whether a synchronous call of that size is cut
+// A queue of the default batch size: the first batch after its creation or a flush holds 1e9 cells, each next one up to
+// twice the last's, up to 2e11, so that the device starts while the caller still pushes; with 2e11 from the start, inputs
+// of that size or less were pushed, marshalled, uploaded and computed in turn (regions of workload 4, push to flush: 20
+// regions 1.86 -> 1.65 ms, 100 10.3 -> 8.0, 200 at 7.4e10 cells 31.9 -> 22.6, 400 68.8 -> 44.8; from 5e9 on 1.9, 7.9,
+// 23.1, 45.4; growing 1.5 times 23.1 and 46.2 at 200 and 400, 3 times 24.8 and 50.4).  A batch size that the caller
+// names holds from the first batch on.
+constexpr int64_t kQueueFirstCells = (int64_t)1e9;
 int queue_open(ghmm_ctx *ctx, int64_t batch_cells, ghmm_queue **out, const ghmm_read_prep *raw_prep = nullptr,
                const RouteBound *bound = nullptr);
 void queue_close(ghmm_queue *q);

@@ -330,7 +330,8 @@ int ghmm_pd_batch_create_raw(ghmm_ctx *ctx, const ghmm_pd_raw_region *regions, i
  * (PH/VectorLoglessPairHMM.java:138, called once per region from HC/HaplotypeCallerEngine.java:734-918
  * through PairHMMLikelihoodCalculationEngine.computeReadLikelihoods); the queue is what a caller puts in
  * front of it to batch regions.
- *   ghmm_queue_create: a queue on ctx; batches are launched once they hold batch_cells cells (0: 2e11).
+ *   ghmm_queue_create: a queue on ctx; batches are launched once they hold batch_cells cells (0: 1e9 cells for the
+ *                      first batch of a queue or after a flush, each next one twice the last's, up to 2e11).
  *   ghmm_queue_push:   copy n_regions regions into the open batch before returning, so the caller may
  *                      reuse its arrays; their read-major results go to out (as ghmm_compute_regions), which
  *                      must stay valid until ghmm_queue_flush returns.  Input errors are reported by this
