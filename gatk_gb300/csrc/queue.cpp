@@ -309,7 +309,7 @@ std::unique_ptr<QueueUnit> borrowed_unit(const Source &src, int64_t g0, int64_t 
 
 // A call runs as a pipeline from 250,000 pairs on, where its marshal, upload and results, which go with the pairs and
 // their bytes, cost more than what the extra batches' launches and kernel tails do.  End to end, one batch against the
-// pipeline: workload 0 at 400 regions (205,000 pairs) 4.58 and 4.55 ms, at 600 6.60 and 5.74, at 5,000 56.8 and 34.8;
+// pipeline: workload 0 at 400 regions (205,000 pairs) 4.58 and 4.55 ms, at 600 6.60 and 5.74, at 5,000 56.8 and 33.9;
 // workload 1 at 150 regions (200,000 pairs) 5.84 and 5.85 ms, at 300 10.3 and 9.7, at 1,000 34.6 and 29.2; workload 3
 // at 40,000 regions (320,000 pairs) 26.1 and 22.0.  Of few long pairs only inputs of 1.5e11 cells are cut, which bounds
 // a batch's memory: workload 2 at 100 regions (35,000 pairs, 1.1e11 cells) takes 1,011 and 1,024 ms.
@@ -317,18 +317,19 @@ bool pipelines(int64_t cells, int64_t pairs, int64_t regions) {
     return regions >= 4 && (pairs >= kPipelineMinPairs || cells >= kPipelineMinCells);
 }
 
-// Region cuts [0 = c_0 < c_1 < ... = G] of a pipelined call over regions of the given cells: a small chunk first, each
-// next one 2.5 times the last up to 1/3 of the cells, so the first marshal the device waits for stays short.  The
-// first chunk is 1/8 of the cells below 1e11 and 1/16 above, where an eighth is long enough to wait for (end to end
-// with 1/8 and 1/16: workload 0 at 1,200 regions, 2.8e10 cells, 9.1 and 9.7 ms, at 5,000, 1.15e11, 34.8 and 34.0;
-// workload 1 at 400 regions, 4e10, 12.2 and 12.7, at 3,000, 3.2e11, 81.6 and 80.1, at 6,000 162.2 and 158.2).  No cut
-// leaves fewer than 8 regions behind it.
-std::vector<int64_t> growing_cuts(const std::vector<int64_t> &cells) {
-    const int64_t G = (int64_t)cells.size();
+int64_t sum_cells(const std::vector<int64_t> &cells) {
     int64_t total = 0;
     for (int64_t c : cells) total += c;
+    return total;
+}
+
+// Region cuts [0 = c_0 < c_1 < ... = G] over regions of the given cells: `first` cells first, each next chunk 2.5 times
+// the last up to 1/3 of all, so the first marshal the device waits for stays short.  No cut leaves fewer than 8 regions
+// behind it.
+std::vector<int64_t> growing_cuts(const std::vector<int64_t> &cells, int64_t first) {
+    const int64_t G = (int64_t)cells.size(), total = sum_cells(cells);
     std::vector<int64_t> cut{0};
-    int64_t target = std::max<int64_t>(total / (total < (int64_t)1e11 ? 8 : 16), 1);
+    int64_t target = std::max<int64_t>(first, 1);
     for (int64_t g0 = 0; g0 < G;) {
         int64_t g1 = g0, c = 0;
         while (g1 < G && (c < target || g1 == g0)) c += cells[(size_t)g1++];
@@ -340,14 +341,19 @@ std::vector<int64_t> growing_cuts(const std::vector<int64_t> &cells) {
     return cut;
 }
 
+// Of a pipelined call: 1/8 of the cells first, at most 8e9, which the device takes 2 ms for (with 1/16 workload 0 at
+// 1,200 regions took 9.7 ms instead of 9.0, workload 4 at 100 regions 19.5 instead of 18.9; without the limit workload 1
+// at 3,000 and 6,000 regions 81.6 and 162.2 ms, with 1/16 82.4 and 156.8, now 81.9 and 154.4; growing two times 155.7).
+std::vector<int64_t> call_cuts(const std::vector<int64_t> &cells) {
+    return growing_cuts(cells, std::min<int64_t>(sum_cells(cells) / 8, (int64_t)8e9));
+}
+
 // Region cuts of a one-shot PD-HMM call.  Below 5e11 cells: three chunks, after 1/8 and 1/2 of the cells, because each
-// chunk's launches, graph capture and kernel tails cost a fixed time.  Above: growing_cuts.  No cut leaves fewer than
-// 8 regions behind it.
+// chunk's launches, graph capture and kernel tails cost a fixed time.  Above: growing_cuts from 1/16 of the cells.  No
+// cut leaves fewer than 8 regions behind it.
 std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells) {
-    const int64_t G = (int64_t)cells.size();
-    int64_t total = 0;
-    for (int64_t c : cells) total += c;
-    if (total >= kPipelineLargeCells) return growing_cuts(cells);
+    const int64_t G = (int64_t)cells.size(), total = sum_cells(cells);
+    if (total >= kPipelineLargeCells) return growing_cuts(cells, total / 16);
     std::vector<int64_t> cut{0};
     const int64_t marks[2] = {total / 8, total / 2};
     int64_t c = 0;
@@ -386,7 +392,7 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
         first_read.assign((size_t)G + 1, 0);
         for (int64_t g = 0; g < G; g++) first_read[(size_t)g + 1] = first_read[(size_t)g] + src.regions[g].n_reads;
     }
-    const std::vector<int64_t> cut = growing_cuts(reg_cells);
+    const std::vector<int64_t> cut = call_cuts(reg_cells);
     for (size_t i = 0; i + 1 < cut.size(); i++) {
         const int64_t g0 = cut[i], g1 = cut[i + 1];
         int64_t c = 0;

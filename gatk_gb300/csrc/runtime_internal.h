@@ -370,7 +370,6 @@ int compute_sync(ghmm_ctx *ctx, const Source &src, double *out);
 // one-shot PD-HMM calls: cells from which they run in chunks, and from which these are growing ones
 constexpr int64_t kPdPipelineMinCells = (int64_t)2e9;
 constexpr int64_t kPipelineLargeCells = (int64_t)5e11;
-std::vector<int64_t> growing_cuts(const std::vector<int64_t> &cells);   // region cuts of a pipelined call
 std::vector<int64_t> pipeline_cuts(const std::vector<int64_t> &cells);  // region cuts of a one-shot PD-HMM call
 
 // pd_host.cpp
