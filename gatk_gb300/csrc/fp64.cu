@@ -39,7 +39,6 @@
 
 #include "../../include/ghmm.h"
 #include "ghmm_internal.h"
-#include "warp_list.cuh"
 
 namespace ghmm {
 namespace {

@@ -20,7 +20,7 @@
 //    (K >= 2).  Each read is followed by two accumulator rows that sum the last row over
 //    the haplotype (row_coef), and padded at the top with "dummy" rows that reproduce the row-0 boundary, so
 //    the accumulator rows always sit in lane 31's last two slots.  Reads longer than 32*K rows run
-//    as several strips whose boundary row goes through per-warp global scratch.  Each row's states are
+//    as several strips whose boundary row goes through per-warp global scratch (and a ring in shared memory).  Each row's states are
 //    rescaled so a cell costs 5 FMA-pipe operations instead of 8: with a_0 = 1, a_i = a_{i-1} / MM_i,
 //       M~ = a_i M,   I~ = (a_{i-1} / MI_i) I,   D~ = (a_i / MD_i) D,
 //    the recurrence becomes

@@ -1,4 +1,4 @@
-// warp_list.cuh -- how a grid of warps takes the entries of a work list (kernels.cu, pd.cu).  Internal linkage: each
+// warp_list.cuh -- how a grid of warps takes the entries of a work list (pd.cu).  Internal linkage: each
 // translation unit that includes it gets its own copy.
 #pragma once
 #include <cuda_runtime.h>
