@@ -1,44 +1,49 @@
 // host_pool.cpp -- see host_pool.h.
 #include "host_pool.h"
 
-#include <unistd.h>
+#include <pthread.h>
 
 #include <algorithm>
 
 namespace ghmm {
 
 namespace {
-std::mutex g_mu;
-std::shared_ptr<HostPool> g_pool;
-int g_refs = 0;
+// The process's pool.  Never destroyed itself: at exit the threads may still sleep in the pool.
+struct Shared {
+    std::mutex mu;
+    std::shared_ptr<HostPool> pool;
+    int refs = 0;
+};
+Shared *g_shared = new Shared;
+
+// In a forked child the pool's threads do not exist: its mutexes may be held, and its condition variables have waiters,
+// for good, so destroying them would wait for ever.  The child leaves all of it as it is and starts without a pool.
+void abandon_in_child() { g_shared = new Shared; }
+[[maybe_unused]] const int g_registered = pthread_atfork(nullptr, nullptr, abandon_in_child);
 }  // namespace
 
 void HostPool::retain() {
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (g_refs++ == 0) g_pool.reset(new HostPool());
+    std::lock_guard<std::mutex> lk(g_shared->mu);
+    if (g_shared->refs++ == 0) g_shared->pool.reset(new HostPool());
 }
 
 void HostPool::release() {
     std::shared_ptr<HostPool> last;
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (--g_refs == 0) last.swap(g_pool);
+    std::lock_guard<std::mutex> lk(g_shared->mu);
+    if (g_shared->refs > 0 && --g_shared->refs == 0) last.swap(g_shared->pool);  // (0: a context of the parent process)
 }
 
 std::shared_ptr<HostPool> HostPool::get() {
-    std::lock_guard<std::mutex> lk(g_mu);
-    return g_pool && g_pool->pid_ == (int)getpid() ? g_pool : nullptr;
+    std::lock_guard<std::mutex> lk(g_shared->mu);
+    return g_shared->pool;
 }
 
-HostPool::HostPool() : pid_((int)getpid()) {
+HostPool::HostPool() {
     const int n = std::max(1, (int)std::thread::hardware_concurrency()) - 1;
     for (int i = 0; i < n; i++) threads_.emplace_back([this] { loop(); });
 }
 
 HostPool::~HostPool() {
-    if (pid_ != (int)getpid()) {  // the threads exist in the parent process only
-        for (auto &t : threads_) t.detach();
-        return;
-    }
     {
         std::lock_guard<std::mutex> lk(mu_);
         stop_ = true;

@@ -17,7 +17,7 @@ public:
     // One reference per open context (ghmm_initialize / ghmm_done); the last one ends the threads, one per core but one.
     static void retain();
     static void release();
-    // The live pool, or null: no context is open, or this process was forked from the one that started the threads.
+    // The live pool, or null: no context of this process is open (a forked child starts without the parent's).
     static std::shared_ptr<HostPool> get();
 
     // work() on the calling thread and on up to `helpers` pool threads at once; returns when all of them have returned.
@@ -41,7 +41,6 @@ private:
     std::deque<Job *> jobs_;
     std::vector<std::thread> threads_;
     bool stop_ = false;
-    int pid_ = 0;
 };
 
 }  // namespace ghmm

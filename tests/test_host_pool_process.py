@@ -1,0 +1,96 @@
+"""The host threads' pool by itself, in small programs built from host_pool.cpp: what a process that forks, ends or has
+few threads to give does with it."""
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "gatk_gb300", "csrc")
+
+HEAD = r"""
+#include <sys/wait.h>
+#include <unistd.h>
+
+#include <atomic>
+#include <cstdio>
+#include <csignal>
+#include <cstdlib>
+#include <thread>
+
+#include "host_pool.h"
+
+using ghmm::HostPool;
+
+// the exit status of a child that runs f, -1 when it has not ended after five seconds
+template <typename F>
+int child(F f) {
+    fflush(nullptr);
+    const pid_t pid = fork();
+    if (pid == 0) {
+        f();
+        exit(0);
+    }
+    for (int i = 0; i < 5000; i++) {
+        int status = 0;
+        if (waitpid(pid, &status, WNOHANG) == pid) return WIFEXITED(status) ? WEXITSTATUS(status) : -2;
+        usleep(1000);
+    }
+    kill(pid, 9);
+    waitpid(pid, nullptr, 0);
+    return -1;
+}
+// 0 when a loop over the pool, or on the calling thread where there is none, does all of its work
+int loop() {
+    std::atomic<int> next{0}, done{0};
+    const std::function<void()> work = [&] {
+        while (next.fetch_add(1) < 1000) done++;
+    };
+    if (const auto pool = HostPool::get())
+        pool->run(3, work);
+    else
+        work();
+    return done.load() == 1000 ? 0 : 7;
+}
+"""
+
+
+def _run(tmp_path, main, flags=(), timeout=120):
+    src, exe = tmp_path / "prog.cpp", tmp_path / "prog"
+    src.write_text(HEAD + main)
+    subprocess.run([os.environ.get("CXX", "g++"), "-O1", "-std=c++17", "-pthread", *flags, "-I", CSRC, str(src),
+                    os.path.join(CSRC, "host_pool.cpp"), "-o", str(exe)], check=True, capture_output=True)
+    return subprocess.run([str(exe)], capture_output=True, text=True, timeout=timeout)
+
+
+@pytest.mark.parametrize("ends", ["", "HostPool::release();", "HostPool::release(); HostPool::release();",
+                                  "if (HostPool::get()) exit(8); if (loop()) exit(9);"])
+def test_forked_child_ends(tmp_path, ends):
+    """A child of a process with an open pool, whose threads sleep, ends by exit(), also after giving the pool up."""
+    r = _run(tmp_path, "int main() { HostPool::retain(); loop(); usleep(20000); const int rc = child([] { %s });"
+                       "printf(\"%%d\", rc); return loop(); }" % ends)
+    assert (r.returncode, r.stdout) == (0, "0")
+
+
+def test_child_forked_while_the_pool_is_in_use(tmp_path):
+    """Another thread may hold any of the pool's locks at the moment of the fork."""
+    r = _run(tmp_path, r"""
+int main() {
+    std::atomic<bool> stop{false};
+    std::thread other([&] { while (!stop) { HostPool::retain(); loop(); HostPool::release(); } });
+    std::thread third([&] { while (!stop) HostPool::get(); });
+    int bad = 0;
+    for (int i = 0; i < 200 && !bad; i++) bad = child([] { HostPool::get(); if (loop()) exit(9); });
+    stop = true;
+    other.join();
+    third.join();
+    printf("%d", bad);
+    return 0;
+}""")
+    assert (r.returncode, r.stdout) == (0, "0")
+
+
+def test_process_ends_with_the_pool_open(tmp_path):
+    r = _run(tmp_path, "int main() { HostPool::retain(); return loop(); }")
+    assert r.returncode == 0
