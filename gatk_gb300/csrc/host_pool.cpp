@@ -68,13 +68,14 @@ void HostPool::loop() {
 }
 
 void HostPool::run(int helpers, const std::function<void()> &work) {
-    Job job{&work, std::min(helpers, (int)threads_.size())};
-    if (job.tickets > 0) {
+    const int tickets = std::min(helpers, (int)threads_.size());  // (job's go down as helpers join)
+    Job job{&work, tickets};
+    if (tickets > 0) {
         {
             std::lock_guard<std::mutex> lk(mu_);
             jobs_.push_back(&job);
         }
-        if (job.tickets == 1)
+        if (tickets == 1)
             wake_.notify_one();
         else
             wake_.notify_all();

@@ -94,3 +94,29 @@ int main() {
 def test_process_ends_with_the_pool_open(tmp_path):
     r = _run(tmp_path, "int main() { HostPool::retain(); return loop(); }")
     assert r.returncode == 0
+
+
+THREADS = r"""
+int main() {
+    HostPool::retain();
+    std::atomic<int> bad{0};
+    const std::function<void()> user = [&] { for (int i = 0; i < 300; i++) bad += loop(); };
+    std::thread a(user), b(user);
+    user();
+    a.join();
+    b.join();
+    HostPool::release();
+    return bad.load();
+}"""
+
+
+def test_loops_of_several_threads_have_no_data_race(tmp_path):
+    """ThreadSanitizer over loops of three threads at once (where the compiler's runs on this machine)."""
+    probe = tmp_path / "probe.cpp"
+    probe.write_text("int main() {}")
+    exe = str(tmp_path / "probe")
+    if subprocess.run([os.environ.get("CXX", "g++"), "-fsanitize=thread", str(probe), "-o", exe],
+                      capture_output=True).returncode or subprocess.run([exe], capture_output=True).returncode:
+        pytest.skip("no ThreadSanitizer")
+    r = _run(tmp_path, THREADS, flags=("-fsanitize=thread", "-g"))
+    assert r.returncode == 0 and "data race" not in r.stderr, r.stderr[:2000]
