@@ -4,6 +4,7 @@
 #include <pthread.h>
 
 #include <algorithm>
+#include <system_error>
 
 namespace ghmm {
 
@@ -22,9 +23,11 @@ void abandon_in_child() { g_shared = new Shared; }
 [[maybe_unused]] const int g_registered = pthread_atfork(nullptr, nullptr, abandon_in_child);
 }  // namespace
 
-void HostPool::retain() {
+void HostPool::retain(int threads) {
     std::lock_guard<std::mutex> lk(g_shared->mu);
-    if (g_shared->refs++ == 0) g_shared->pool.reset(new HostPool());
+    if (!g_shared->pool) g_shared->pool.reset(new HostPool());
+    g_shared->refs++;
+    g_shared->pool->grow(threads - 1);
 }
 
 void HostPool::release() {
@@ -38,9 +41,12 @@ std::shared_ptr<HostPool> HostPool::get() {
     return g_shared->pool;
 }
 
-HostPool::HostPool() {
-    const int n = std::max(1, (int)std::thread::hardware_concurrency()) - 1;
-    for (int i = 0; i < n; i++) threads_.emplace_back([this] { loop(); });
+void HostPool::grow(int n) {
+    std::lock_guard<std::mutex> lk(mu_);
+    try {
+        while ((int)threads_.size() < n) threads_.emplace_back([this] { loop(); });
+    } catch (const std::system_error &) {  // no more threads to be had: the loops run on those there are
+    }
 }
 
 HostPool::~HostPool() {
@@ -68,13 +74,14 @@ void HostPool::loop() {
 }
 
 void HostPool::run(int helpers, const std::function<void()> &work) {
-    const int tickets = std::min(helpers, (int)threads_.size());  // (job's go down as helpers join)
-    Job job{&work, tickets};
+    int tickets;  // (job's go down as helpers join)
+    Job job{&work, 0};
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        job.tickets = tickets = std::min(helpers, (int)threads_.size());
+        if (tickets > 0) jobs_.push_back(&job);
+    }
     if (tickets > 0) {
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            jobs_.push_back(&job);
-        }
         if (tickets == 1)
             wake_.notify_one();
         else

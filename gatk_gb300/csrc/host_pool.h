@@ -14,8 +14,10 @@ namespace ghmm {
 
 class HostPool {
 public:
-    // One reference per open context (ghmm_initialize / ghmm_done); the last one ends the threads, one per core but one.
-    static void retain();
+    // One reference per open context (ghmm_initialize / ghmm_done), with the threads its loops may run on, the caller's
+    // one of them: the pool has as many as the context with the most asks for (or as could be started) until the last
+    // reference goes.
+    static void retain(int threads);
     static void release();
     // The live pool, or null: no context of this process is open (a forked child starts without the parent's).
     static std::shared_ptr<HostPool> get();
@@ -33,7 +35,8 @@ private:
         int tickets;     // helpers that may still join
         int active = 0;  // helpers inside work()
     };
-    HostPool();
+    HostPool() = default;
+    void grow(int n);
     void loop();
 
     std::mutex mu_;

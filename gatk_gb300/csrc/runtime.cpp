@@ -218,7 +218,7 @@ int ghmm_initialize(const ghmm_args *args, ghmm_ctx **out) {
     ctx->tables.lm2m64 = dt->lm2m64;
     static std::atomic<uint64_t> next_id{1};
     ctx->id = next_id.fetch_add(1);
-    HostPool::retain();
+    HostPool::retain(hw_threads(a.max_threads));
     ctx->alive = true;
     *out = ctx;
     return GHMM_OK;

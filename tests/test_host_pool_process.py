@@ -68,7 +68,7 @@ def _run(tmp_path, main, flags=(), timeout=120):
                                   "if (HostPool::get()) exit(8); if (loop()) exit(9);"])
 def test_forked_child_ends(tmp_path, ends):
     """A child of a process with an open pool, whose threads sleep, ends by exit(), also after giving the pool up."""
-    r = _run(tmp_path, "int main() { HostPool::retain(); loop(); usleep(20000); const int rc = child([] { %s });"
+    r = _run(tmp_path, "int main() { HostPool::retain(4); loop(); usleep(20000); const int rc = child([] { %s });"
                        "printf(\"%%d\", rc); return loop(); }" % ends)
     assert (r.returncode, r.stdout) == (0, "0")
 
@@ -78,7 +78,7 @@ def test_child_forked_while_the_pool_is_in_use(tmp_path):
     r = _run(tmp_path, r"""
 int main() {
     std::atomic<bool> stop{false};
-    std::thread other([&] { while (!stop) { HostPool::retain(); loop(); HostPool::release(); } });
+    std::thread other([&] { while (!stop) { HostPool::retain(4); loop(); HostPool::release(); } });
     std::thread third([&] { while (!stop) HostPool::get(); });
     int bad = 0;
     for (int i = 0; i < 200 && !bad; i++) bad = child([] { HostPool::get(); if (loop()) exit(9); });
@@ -92,13 +92,13 @@ int main() {
 
 
 def test_process_ends_with_the_pool_open(tmp_path):
-    r = _run(tmp_path, "int main() { HostPool::retain(); return loop(); }")
+    r = _run(tmp_path, "int main() { HostPool::retain(4); return loop(); }")
     assert r.returncode == 0
 
 
 THREADS = r"""
 int main() {
-    HostPool::retain();
+    HostPool::retain(4);
     std::atomic<int> bad{0};
     const std::function<void()> user = [&] { for (int i = 0; i < 300; i++) bad += loop(); };
     std::thread a(user), b(user);
@@ -120,3 +120,51 @@ def test_loops_of_several_threads_have_no_data_race(tmp_path):
         pytest.skip("no ThreadSanitizer")
     r = _run(tmp_path, THREADS, flags=("-fsanitize=thread", "-g"))
     assert r.returncode == 0 and "data race" not in r.stderr, r.stderr[:2000]
+
+
+def test_threads_are_those_the_contexts_ask_for(tmp_path):
+    r = _run(tmp_path, r"""
+#include <filesystem>
+int tasks() {
+    int n = 0;
+    for (const auto &e : std::filesystem::directory_iterator("/proc/self/task")) n += e.exists();
+    return n;
+}
+int main() {
+    int bad = 0;
+    HostPool::retain(1);
+    printf("%d ", tasks());
+    bad += loop();
+    HostPool::retain(3);
+    printf("%d ", tasks());
+    bad += loop();
+    HostPool::retain(2);
+    printf("%d ", tasks());
+    for (int i = 0; i < 3; i++) HostPool::release();
+    printf("%d", tasks());
+    return bad;
+}""")
+    assert (r.returncode, r.stdout) == (0, "1 3 3 1")
+
+
+def test_threads_that_cannot_be_started(tmp_path):
+    """An address space with room for two or three stacks: the loops run on the threads there are."""
+    r = _run(tmp_path, r"""
+#include <sys/resource.h>
+int main() {
+    rlimit stack{}, lim{};
+    getrlimit(RLIMIT_STACK, &stack);  // the size of a thread's stack
+    long pages = 0;
+    FILE *f = fopen("/proc/self/statm", "r");
+    if (stack.rlim_cur > ((rlim_t)1 << 30) || !f || fscanf(f, "%ld", &pages) != 1) return 77;
+    getrlimit(RLIMIT_AS, &lim);
+    lim.rlim_cur = (rlim_t)pages * sysconf(_SC_PAGESIZE) + 3 * stack.rlim_cur;
+    setrlimit(RLIMIT_AS, &lim);
+    HostPool::retain(64);
+    int bad = loop();
+    HostPool::release();
+    return bad;
+}""")
+    if r.returncode == 77:
+        pytest.skip("no limit on a thread's stack")
+    assert r.returncode == 0
