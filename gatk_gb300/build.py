@@ -30,7 +30,8 @@ CPP_SOURCES = ["runtime.cpp", "host_pool.cpp", "batch.cpp", "queue.cpp", "pd_hos
                "sw_host.cpp", "multi.cpp"]
 SYNTH_SOURCES = ["synth.cpp"]
 SYNTH_LIB = os.path.join(OUT_DIR, "libghmm_synth.so")
-HEADERS = ["fp32_rows.cuh", "warp_list.cuh", "ghmm_internal.h", "runtime_internal.h", "tables.h", "str_analyzer.h", "host_util.h", "host_pool.h"]
+HEADERS = ["fp32_rows.cuh", "warp_list.cuh", "ghmm_internal.h", "runtime_internal.h", "tables.h", "str_analyzer.h", "host_util.h", "host_pool.h",
+           "spare_slots.h"]
 
 
 def nvcc() -> str:

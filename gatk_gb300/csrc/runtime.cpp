@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "runtime_internal.h"
+#include "spare_slots.h"
 
 namespace ghmm {
 std::atomic<int64_t> g_refuse_allocations{0};
@@ -59,28 +60,17 @@ int cuda_fail(ghmm_ctx *ctx, cudaError_t e, const char *what) {
 // regions otherwise allocates and frees some thirty pinned and device buffers each time (150 regions: 5 of the 18 ms
 // from raw reads to cigars).  At most one batch a context, of at most kSpareBytes; given back when the context closes,
 // and by any allocation of the process that fails (release_spare_batches).
-struct SpareBatch {
-    uint64_t ctx_id;
-    int device;
-    ghmm_batch *b;
-};
 constexpr size_t kSpareBytes = (size_t)1 << 30;
-std::mutex g_spare_mu;
-std::vector<SpareBatch> g_spares;
+SpareSlots<ghmm_batch> g_spares;
 
-ghmm_batch *take_spare(uint64_t ctx_id) {
-    std::lock_guard<std::mutex> lk(g_spare_mu);
-    for (size_t i = 0; i < g_spares.size(); i++)
-        if (g_spares[i].ctx_id == ctx_id) {
-            ghmm_batch *b = g_spares[i].b;
-            g_spares.erase(g_spares.begin() + (ptrdiff_t)i);
-            return b;
-        }
-    return nullptr;
+void free_spare(ghmm_batch *b) {
+    if (!b) return;
+    b->release();
+    delete b;
 }
 
 ghmm_batch *new_batch(ghmm_ctx *ctx) {
-    ghmm_batch *b = take_spare(ctx->id);
+    ghmm_batch *b = g_spares.take(ctx->id);
     if (!b) b = new ghmm_batch();
     b->ctx_id = ctx->id;
     return b;
@@ -90,28 +80,21 @@ ghmm_batch *new_batch(ghmm_ctx *ctx) {
 bool keep_spare(ghmm_ctx *ctx, ghmm_batch *b) {
     if (b->buffer_bytes() > kSpareBytes) return false;
     b->recycle();
-    if (ghmm_batch *old = take_spare(ctx->id)) {
-        old->release();
-        delete old;
-    }
-    std::lock_guard<std::mutex> lk(g_spare_mu);
-    g_spares.push_back(SpareBatch{ctx->id, ctx->device, b});
+    free_spare(g_spares.put(ctx->id, ctx->device, b));
     return true;
 }
 
 }  // namespace rt
 
 bool release_spare_batches() {
-    std::lock_guard<std::mutex> lk(rt::g_spare_mu);
-    if (rt::g_spares.empty()) return false;
+    const auto spares = rt::g_spares.take_all();
+    if (spares.empty()) return false;
     int device = 0;
     cudaGetDevice(&device);
-    for (auto &s : rt::g_spares) {
+    for (const auto &s : spares) {
         cudaSetDevice(s.device);
-        s.b->release();
-        delete s.b;
+        rt::free_spare(s.kept);
     }
-    rt::g_spares.clear();
     cudaSetDevice(device);
     return true;
 }
@@ -316,10 +299,7 @@ int ghmm_done(ghmm_ctx *ctx) {
     if (ctx->pipe) queue_close(ctx->pipe);
     ctx->pipe = nullptr;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    if (ghmm_batch *spare = take_spare(ctx->id)) {
-        spare->release();
-        delete spare;
-    }
+    free_spare(g_spares.take(ctx->id));
     ctx->scratch_batch.release();
     for (auto &pb : ctx->pd_batch) pb.release();
     ctx->calib_scratch.release();
