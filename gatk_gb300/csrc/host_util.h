@@ -31,11 +31,24 @@ struct NvtxRange {
     NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
-// Test hook (ghmm_debug_inject): the number of device allocations still to be refused as out of memory
-extern std::atomic<int64_t> g_refuse_allocations;
+// Test hooks (ghmm_debug_inject): the number of device allocations still to be refused as out of memory, and of device
+// and pinned ones still to find the memory taken up
+extern std::atomic<int64_t> g_refuse_allocations, g_full_allocations;
 
 // Frees the buffers that contexts keep of destroyed batches (runtime.cpp); false when there were none.
 bool release_spare_batches();
+
+// alloc(); where it finds no memory, once more after the buffers that contexts keep were given back.
+template <typename F>
+inline cudaError_t alloc_or_trim(F alloc) {
+    const bool full = g_full_allocations.load(std::memory_order_relaxed) > 0 && g_full_allocations.fetch_sub(1) > 0;
+    cudaError_t e = full ? cudaErrorMemoryAllocation : alloc();
+    if (e == cudaErrorMemoryAllocation && release_spare_batches()) {
+        cudaGetLastError();  // the failed attempt's
+        e = alloc();
+    }
+    return e;
+}
 
 template <typename T>
 struct DevBuf {
@@ -51,11 +64,7 @@ struct DevBuf {
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        cudaError_t e = cudaMalloc(&p, want * sizeof(T));
-        if (e == cudaErrorMemoryAllocation && release_spare_batches()) {
-            cudaGetLastError();  // the failed attempt's
-            e = cudaMalloc(&p, want * sizeof(T));
-        }
+        const cudaError_t e = alloc_or_trim([&] { return cudaMalloc(&p, want * sizeof(T)); });
         if (e == cudaSuccess) cap = want;
         return e;
     }
@@ -76,11 +85,7 @@ struct HostBuf {  // pinned
         if (p) cudaFreeHost(p);
         p = nullptr;
         cap = 0;
-        cudaError_t e = cudaMallocHost(&p, want * sizeof(T));
-        if (e == cudaErrorMemoryAllocation && release_spare_batches()) {
-            cudaGetLastError();
-            e = cudaMallocHost(&p, want * sizeof(T));
-        }
+        const cudaError_t e = alloc_or_trim([&] { return cudaMallocHost(&p, want * sizeof(T)); });
         if (e == cudaSuccess) cap = want;
         return e;
     }

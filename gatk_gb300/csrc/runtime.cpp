@@ -24,7 +24,7 @@
 #include "spare_slots.h"
 
 namespace ghmm {
-std::atomic<int64_t> g_refuse_allocations{0};
+std::atomic<int64_t> g_refuse_allocations{0}, g_full_allocations{0};
 }
 
 namespace {
@@ -58,8 +58,9 @@ int cuda_fail(ghmm_ctx *ctx, cudaError_t e, const char *what) {
 
 // The buffers of each open context's last destroyed batch, for its next one: a program that makes a batch per group of
 // regions otherwise allocates and frees some thirty pinned and device buffers each time (150 regions: 5 of the 18 ms
-// from raw reads to cigars).  At most one batch a context, of at most kSpareBytes; given back when the context closes,
-// and by any allocation of the process that fails (release_spare_batches).
+// from raw reads to cigars).  At most one batch a context, of at most kSpareBytes of device and pinned memory together;
+// given back by ghmm_trim, when the context closes, and when an allocation of this library's buffers finds no memory
+// (alloc_or_trim).  Other allocators of the process do not know of it: their callers use ghmm_trim.
 constexpr size_t kSpareBytes = (size_t)1 << 30;
 SpareSlots<ghmm_batch> g_spares;
 
@@ -128,6 +129,7 @@ int ghmm_debug_inject(ghmm_ctx *ctx, int32_t kind, int64_t arg) {
     if (arg < 0) return fail(ctx, GHMM_ERR_ARG, "negative injection argument");
     switch (kind) {
         case GHMM_INJECT_REFUSE_ALLOCATIONS: ghmm::g_refuse_allocations.store(arg); return GHMM_OK;
+        case GHMM_INJECT_FULL_MEMORY: ghmm::g_full_allocations.store(arg); return GHMM_OK;
         case GHMM_INJECT_FP64_RERUN_EVERY: ctx->debug_force_rerun = arg; return GHMM_OK;
         default: return fail(ctx, GHMM_ERR_ARG, "unknown injection");
     }
@@ -609,6 +611,17 @@ int ghmm_calib_fold(ghmm_ctx *ctx, const int64_t *d_index, int64_t n, const floa
     const int e = launch_calib_fold(d_index, n, d_grad_open, d_grad_cont, (int)rows, d_table, ctx->sm_count,
                                     (cudaStream_t)stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "calibration fold launch");
+    return GHMM_OK;
+}
+
+int ghmm_trim(ghmm_ctx *ctx, int64_t *freed) {
+    if (!ctx || !ctx->alive) return GHMM_ERR_STATE;
+    ghmm_batch *spare = g_spares.take(ctx->id);
+    if (freed) *freed = spare ? (int64_t)spare->buffer_bytes() : 0;
+    if (spare) {
+        GHMM_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
+        free_spare(spare);
+    }
     return GHMM_OK;
 }
 

@@ -28,6 +28,7 @@ MODE_PD = 3
 MODE_PD_FP32 = 4
 INJECT_REFUSE_ALLOCATIONS = 1
 INJECT_FP64_RERUN_EVERY = 2
+INJECT_FULL_MEMORY = 3
 CALIB_FOLD_ROWS = 2048  # GHMM_CALIB_FOLD_ROWS
 FP64_RESCALED_FLOOR = -560.0  # GHMM_FP64_RESCALED_FLOOR
 MODE_PLAIN_FP64 = 2
@@ -221,6 +222,7 @@ _SIGS = {
     "ghmm_batch_results": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, _f64p]),
     "ghmm_batch_stats": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(Stats)]),
     "ghmm_batch_destroy": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
+    "ghmm_trim": (ctypes.c_int, [ctypes.c_void_p, _i64p]),
     "ghmm_compute_regions_raw": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
                                                 ctypes.POINTER(ReadPrep), _f64p]),
     "ghmm_batch_create_raw": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,

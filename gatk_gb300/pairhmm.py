@@ -283,6 +283,12 @@ class Engine:
     def stream_handle(self) -> int:
         return int(self.L.ghmm_stream(self._ctx.h) or 0)
 
+    def trim(self) -> int:
+        """Free the buffers kept of the last destroyed batch; their bytes (device and pinned memory)."""
+        freed = ctypes.c_int64(0)
+        native.check(self.L.ghmm_trim(self._ctx.h, ctypes.byref(freed)), self._ctx.h)
+        return freed.value
+
     def compute(self, wl: Workload, via_regions: bool = False) -> np.ndarray:
         """Upload + forward + download (host buffers in, host results out)."""
         out = np.empty(wl.n_pairs, dtype=np.float64)

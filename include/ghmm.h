@@ -190,13 +190,18 @@ int ghmm_last_error(const ghmm_ctx *ctx, char *buf, size_t buf_len);
  * context's internal queue, so that marshalling overlaps the kernels; the results are the same. */
 int ghmm_compute_regions(ghmm_ctx *ctx, const ghmm_region *regions, int32_t n_regions, double *out);
 
-/* Device-resident batches: marshal + upload once, run the forward many times, download. */
+/* Device-resident batches: marshal + upload once, run the forward many times, download.
+ * ghmm_batch_destroy keeps the buffers of the context's last destroyed batch for its next one, up to 1 GiB of device and
+ * pinned memory together.  They are freed by ghmm_trim (*freed, unless NULL: their bytes), by ghmm_done, and when an
+ * allocation of this library finds no memory; a program whose other libraries allocate on the same device calls ghmm_trim
+ * before they need it. */
 int ghmm_batch_create(ghmm_ctx *ctx, const ghmm_region *regions, int32_t n_regions, ghmm_batch **batch);
 int ghmm_batch_create_flat(ghmm_ctx *ctx, const ghmm_flat *flat, ghmm_batch **batch);
 int ghmm_batch_forward(ghmm_ctx *ctx, ghmm_batch *batch, int32_t mode);
 int ghmm_batch_results(ghmm_ctx *ctx, ghmm_batch *batch, double *out);
 int ghmm_batch_stats(ghmm_ctx *ctx, const ghmm_batch *batch, ghmm_stats *stats);
 int ghmm_batch_destroy(ghmm_ctx *ctx, ghmm_batch *batch);
+int ghmm_trim(ghmm_ctx *ctx, int64_t *freed);
 
 /* The step after the likelihoods, fused on the device over a batch's last forward: per read, every haplotype
  * likelihood below best + cap is raised to best + cap (AlleleLikelihoods.normalizeLikelihoods,
@@ -376,12 +381,15 @@ int ghmm_queue_push_raw(ghmm_queue *queue, const ghmm_raw_region *regions, int32
 /* Failure injection for tests, all on the host side (nothing faults, traps or stalls a GPU):
  *   GHMM_INJECT_REFUSE_ALLOCATIONS: the next arg device allocations of the process fail as out of memory, so the
  *                                   calls that need them return GHMM_ERR_NOMEM and the context stays usable;
+ *   GHMM_INJECT_FULL_MEMORY:        the next arg device or pinned allocations of the process's batches find no memory
+ *                                   until the buffers kept of destroyed batches (ghmm_batch_destroy) are freed;
  *   GHMM_INJECT_FP64_RERUN_EVERY:   every arg-th output of the FP32 pass is treated as an underflow and recomputed
  *                                   in FP64 (batches uploaded after the call; 0 turns it off).
  * Setting the environment variable GHMM_REPORT_UNSUPPORTED (not "0") makes ghmm_load report no usable GPU, as a
  * caller's fallback chain sees it (VectorLoglessPairHMM.java:60-79 -> HardwareFeatureException). */
 #define GHMM_INJECT_REFUSE_ALLOCATIONS 1
 #define GHMM_INJECT_FP64_RERUN_EVERY 2
+#define GHMM_INJECT_FULL_MEMORY 3
 int ghmm_debug_inject(ghmm_ctx *ctx, int32_t kind, int64_t arg);
 
 /* Measured FP32 FMA-pipe peak of the device in TFLOP/s (FMA = 2 FLOP): best of a scalar FFMA and a
