@@ -25,41 +25,47 @@ namespace rt {
 
 constexpr size_t kQueueMaxReady = 2;  // sealed batches waiting for the worker before push blocks
 
-// Copy a finished slot's results to its destinations and check them (PairHMM.java:305-306).
-int queue_deliver(ghmm_ctx *ctx, ghmm_batch &b, const QueueUnit &u, int threads) {
-    const double *src = b.h_out.p;
-    std::atomic<int64_t> bad{-1};
-    std::vector<int64_t> base(u.dests.size() + 1, 0);
-    for (size_t i = 0; i < u.dests.size(); i++) base[i + 1] = base[i] + u.dests[i].second;
-    // blocks of at most 1M results, in parallel
-    std::vector<std::pair<size_t, int64_t>> blocks;
-    for (size_t i = 0; i < u.dests.size(); i++)
-        for (int64_t a = 0; a < u.dests[i].second; a += (1 << 20)) blocks.emplace_back(i, a);
+// The results of unit u as blocks of at most 1M, in parallel: f(source, destination, index within the unit, count).
+template <typename F>
+void for_result_blocks(const QueueUnit &u, const double *src, int threads, F f) {
+    struct Block {
+        double *dest;
+        int64_t at, n;
+    };
+    std::vector<Block> blocks;
+    int64_t base = 0;
+    for (const auto &d : u.dests) {
+        for (int64_t a = 0; a < d.second; a += (1 << 20))
+            blocks.push_back(Block{d.first + a, base + a, std::min<int64_t>(d.second - a, 1 << 20)});
+        base += d.second;
+    }
     parallel_for((int64_t)blocks.size(), threads, [&](int64_t k) {
-        const size_t i = blocks[(size_t)k].first;
-        const int64_t a = blocks[(size_t)k].second, e = std::min<int64_t>(u.dests[i].second, a + (1 << 20));
-        const double *s = src + base[i];
-        double *d = u.dests[i].first;
-        for (int64_t j = a; j < e; j++) {
+        const Block &b = blocks[(size_t)k];
+        f(src + b.at, b.dest, b.at, b.n);
+    }, 1);
+}
+
+// Copy a finished unit's results to its destinations and check them (PairHMM.java:305-306).
+int queue_deliver(ghmm_ctx *ctx, const double *src, const QueueUnit &u, int threads) {
+    std::atomic<int64_t> bad{-1};
+    for_result_blocks(u, src, threads, [&](const double *s, double *d, int64_t at, int64_t n) {
+        for (int64_t j = 0; j < n; j++) {
             const double v = s[j];
             d[j] = v;
             if (!(v <= 0.0)) {
                 int64_t expect = -1;
-                bad.compare_exchange_strong(expect, base[i] + j);
+                bad.compare_exchange_strong(expect, at + j);
             }
         }
-    }, 1);
+    });
     if (bad.load() >= 0) {
         char msg[160];
-        snprintf(msg, sizeof msg, "PairHMM log10 likelihood %g at output %lld of a queued batch is not a valid log10 probability",
-                 src[bad.load()], (long long)bad.load());
+        snprintf(msg, sizeof msg, "PairHMM log10 likelihood %g at output %lld%s is not a valid log10 probability",
+                 src[bad.load()], (long long)(u.first_out + bad.load()), u.borrowed ? "" : " of a queued batch");
         return fail(ctx, GHMM_ERR_RESULT, msg);
     }
     return GHMM_OK;
 }
-
-
-
 
 // Worker: marshal + upload (+ read preparation for a raw queue) + launch one unit into slot i (which is free).
 int queue_launch(ghmm_queue *q, int i, QueueUnit &u) {
@@ -97,8 +103,16 @@ int queue_launch(ghmm_queue *q, int i, QueueUnit &u) {
 int queue_retire(ghmm_queue *q, int i) {
     ghmm_ctx *ctx = q->ctx;
     ghmm_batch &b = q->slot[i];
+    const int threads = hw_threads(ctx->max_threads);
     int rc = batch_finish(ctx, b);
-    if (!rc) rc = queue_deliver(ctx, b, *q->inflight[i], hw_threads(ctx->max_threads));
+    const QueueUnit &u = *q->inflight[i];
+    const bool hold = u.borrowed && !q->inputs_ok;
+    if (!rc && hold)
+        for_result_blocks(u, b.h_out.p, threads, [&](const double *s, double *, int64_t at, int64_t n) {
+            memcpy(q->held.get() + u.first_out + at, s, (size_t)n * sizeof(double));
+        });
+    else if (!rc)
+        rc = queue_deliver(ctx, b.h_out.p, u, threads);
     std::lock_guard<std::mutex> lk(q->mu);
     if (!rc) {
         ghmm_queue_info &in = q->info;
@@ -115,6 +129,7 @@ int queue_retire(ghmm_queue *q, int i) {
         in.ms_host_marshal += b.ms_host_copy;
         in.ms_host_tasks += b.ms_host_tasks;
     }
+    if (!rc && hold) q->held_units.push_back(std::move(q->inflight[i]));
     q->inflight[i].reset();
     q->retired++;
     q->cv_done.notify_all();
@@ -185,8 +200,17 @@ void queue_worker(ghmm_queue *q) {
             continue;
         }
         if (!u->borrowed) u->drop_inputs();
+        const bool last = u->last;
         q->inflight[i] = std::move(u);
         q->inflight_seq[i] = ++q->seq;
+        if (last) {  // while it runs, what waited for its input checks
+            q->inputs_ok = true;
+            for (const auto &h : q->held_units) {
+                rc = queue_deliver(q->ctx, q->held.get() + h->first_out, *h, hw_threads(q->ctx->max_threads));
+                if (rc) queue_record_error(q, rc, err);
+            }
+            q->held_units.clear();
+        }
     }
 }
 
@@ -385,6 +409,8 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
         q->error_msg.clear();
         q->mode = ctx->double_precision ? GHMM_MODE_FP64 : GHMM_MODE_FP32_RERUN;
         queue_set_raw(q, mapq ? prep : nullptr, bound);
+        q->held_units.clear();
+        q->inputs_ok = false;
     }
     const int64_t G = src.n_regions;
     std::vector<int64_t> first_read;  // raw reads: the batch's reads' mapping qualities go with the batch
@@ -393,11 +419,19 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
         for (int64_t g = 0; g < G; g++) first_read[(size_t)g + 1] = first_read[(size_t)g] + src.regions[g].n_reads;
     }
     const std::vector<int64_t> cut = call_cuts(reg_cells);
+    const int64_t hold = reg_out[(size_t)cut[cut.size() - 2]];  // results of all units but the last
+    if (hold > q->held_cap) {
+        q->held_cap = 0;
+        q->held.reset(new double[(size_t)hold]);
+        q->held_cap = hold;
+    }
     for (size_t i = 0; i + 1 < cut.size(); i++) {
         const int64_t g0 = cut[i], g1 = cut[i + 1];
         int64_t c = 0;
         for (int64_t g = g0; g < g1; g++) c += reg_cells[(size_t)g];
         auto u = borrowed_unit(src, g0, g1, out + reg_out[(size_t)g0], reg_out[(size_t)g1] - reg_out[(size_t)g0], c);
+        u->first_out = reg_out[(size_t)g0];
+        u->last = i + 2 == cut.size();
         if (mapq) {
             u->mapq.assign(mapq + first_read[(size_t)g0], mapq + first_read[(size_t)g1]);
             u->max_len = max_len;

@@ -243,6 +243,8 @@ struct QueueUnit {
     ghmm_flat flat{};
     std::vector<std::pair<double *, int64_t>> dests;  // output runs in region order
     int64_t cells = 0, n_out = 0, n_regions = 0;
+    int64_t first_out = 0;  // of a synchronous call's unit: its first result within the call
+    bool last = false;      // ... and whether it is the call's last
     std::vector<int32_t> mapq;  // raw queues: mapping quality per read
     int32_t max_len = 0;        // raw queues: longest read
 
@@ -302,6 +304,12 @@ struct ghmm_queue {
     cudaStream_t stream[2]{};
     std::unique_ptr<QueueUnit> inflight[2];
     int64_t inflight_seq[2]{};
+    // synchronous calls: finished units wait here, their results in held, until the call's last unit has passed its
+    // input checks, so that an input error leaves the caller's array as it was
+    std::vector<std::unique_ptr<QueueUnit>> held_units;
+    std::unique_ptr<double[]> held;  // result i of the call at held[i]
+    int64_t held_cap = 0;
+    bool inputs_ok = false;
     int64_t seq = 0;
 };
 

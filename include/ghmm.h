@@ -187,7 +187,8 @@ int ghmm_last_error(const ghmm_ctx *ctx, char *buf, size_t buf_len);
 /* Batcher: many regions in one call (regions of HaplotypeCallerEngine.callRegion batched together).
  * out receives each region's read-major block back to back, in region order.  Inputs of 250,000 pairs or
  * 1.5e11 cells run as a pipeline of batches (the first small, later ones up to a third of the input) on the
- * context's internal queue, so that marshalling overlaps the kernels; the results are the same. */
+ * context's internal queue, so that marshalling overlaps the kernels; the results and the errors are the same: an input
+ * error leaves out as it was, and an invalid result is named by its place in out. */
 int ghmm_compute_regions(ghmm_ctx *ctx, const ghmm_region *regions, int32_t n_regions, double *out);
 
 /* Device-resident batches: marshal + upload once, run the forward many times, download.
