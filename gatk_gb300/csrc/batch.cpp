@@ -314,7 +314,11 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
         };
         std::vector<ReadPair> pairs;
         std::vector<std::pair<int, int64_t>> leftovers;  // (key, read) of the single-strip classes' odd reads
-        std::vector<std::pair<int64_t, int64_t>> chunks;  // haplotype ranges of one task
+        struct Chunk {  // haplotype range of one task
+            int64_t a, e, cols;
+            bool mixed;
+        };
+        std::vector<Chunk> chunks;
         for (int64_t g = G * part / n_parts; g < G * (part + 1) / n_parts; g++) {
             const int64_t h0 = rho[(size_t)g], h1 = rho[(size_t)g + 1];
             const int64_t r0 = rro[(size_t)g], r1 = rro[(size_t)g + 1];
@@ -339,7 +343,7 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
                     key = std::max(2, (rows + 31) / 32);
                 } else {  // fewest strips of at most max_k_multi rows per lane, then the fewest rows per lane
                     ns = (rows + 32 * max_k_multi - 1) / (32 * max_k_multi);
-                    key = std::max(2, (rows + 32 * ns - 1) / (32 * ns)) | 16;
+                    key = std::max(2, (rows + 32 * ns - 1) / (32 * ns)) | kBucketMulti;
                 }
                 // reads are paired only within one (rows per lane, strip count) class
                 groups.emplace_back(((int64_t)key * 4096 + ns) * 100000 + R, r);
@@ -349,14 +353,17 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
             chunks.clear();
             const int64_t even = region_cols / ((region_cols + chunk_cols - 1) / chunk_cols + (region_cols == 0));
             for (int64_t a = h0; a < h1;) {
-                int64_t e = a + 1, cols = hap_off[(size_t)a + 1] - hap_off[(size_t)a];
-                while (e < h1) {
+                int64_t e = a, cols = 0, plain = 0;
+                bool shorts = false;
+                do {
                     const int64_t next = hap_off[(size_t)e + 1] - hap_off[(size_t)e];
-                    if (cols + next > chunk_cols || cols + next / 2 > even) break;
+                    if (e > a && (cols + next > chunk_cols || cols + next / 2 > even)) break;
                     cols += next;
-                    e++;
-                }
-                chunks.emplace_back(a, e);
+                    plain += std::max<int64_t>(next - kShortHapCols, 0);
+                    shorts |= next < kShortHapCols;
+                } while (++e < h1);
+                // (the PD-HMM kernels have one form for all)
+                chunks.push_back(Chunk{a, e, cols, shorts && 4 * plain > cols && !src.region_direct});
                 a = e;
             }
             // neighbours of one class share a task; the single-strip classes' leftovers (one read of each class with
@@ -371,7 +378,7 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
                 int64_t rb = -1;
                 if (i + 1 < groups.size() && groups[i + 1].first / 100000 == cls) rb = groups[i + 1].second;
                 i += (rb >= 0) ? 2 : 1;
-                if (rb < 0 && !(key & 16))
+                if (rb < 0 && !(key & kBucketMulti))
                     leftovers.emplace_back(key, ra);
                 else
                     pairs.push_back(ReadPair{key, ra, rb});
@@ -388,8 +395,8 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
             for (const ReadPair &rp : pairs) {
                 const int key = rp.key;
                 const int64_t ra = rp.a, rb = rp.b;
-                const int K = key & 15;
-                const bool multi = (key & 16) != 0;
+                const int K = bucket_rows(key);
+                const bool multi = (key & kBucketMulti) != 0;
                 const int S = 32 * K;
                 const int Ra = (int)(read_off[(size_t)ra + 1] - read_off[(size_t)ra]);
                 const int Rb = rb >= 0 ? (int)(read_off[(size_t)rb + 1] - read_off[(size_t)rb]) : 0;
@@ -398,17 +405,17 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
                     F32Task t;
                     t.read_a = (int32_t)ra;
                     t.read_b = (int32_t)rb;
-                    t.hap_begin = (int32_t)ch.first;
-                    t.hap_end = (int32_t)ch.second;
+                    t.hap_begin = (int32_t)ch.a;
+                    t.hap_end = (int32_t)ch.e;
                     t.region = (int32_t)g;
                     t.nstrips = (int16_t)nstrips;
                     t.k = (int16_t)K;
                     t.pad_a = nstrips * S - Ra - kAccRows;
                     t.pad_b = rb >= 0 ? nstrips * S - Rb - kAccRows : nstrips * S;
-                    const int64_t cols = hap_off[(size_t)ch.second] - hap_off[(size_t)ch.first];
-                    if (multi) po.max_multi_cols = std::max(po.max_multi_cols, cols);
-                    po.tasks[key].push_back(t);
-                    po.cost[key].push_back((cols + 31) * K * nstrips);
+                    const int task_key = key + (ch.mixed ? kBucketMixed : 0);
+                    if (multi) po.max_multi_cols = std::max(po.max_multi_cols, ch.cols);
+                    po.tasks[task_key].push_back(t);
+                    po.cost[task_key].push_back((ch.cols + 31) * K * nstrips);
                 }
             }
         }
@@ -418,11 +425,19 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
     int64_t total_tasks = 0, max_multi_cols = 0, n_direct = 0, n_direct_exact = 0;
     b.cells_direct = 0;
     std::vector<int64_t> bucket_pos(kNumBucketKeys + 1, 0);
-    for (int key = 0; key < kNumBucketKeys; key++) {
-        int64_t n = 0;
-        for (auto &po : parts) n += (int64_t)po.tasks[key].size();
-        bucket_pos[(size_t)key + 1] = bucket_pos[(size_t)key] + n;
-    }
+    std::vector<int64_t> key_count(kNumBucketKeys, 0);
+    for (int key = 0; key < kNumBucketKeys; key++)
+        for (auto &po : parts) key_count[(size_t)key] += (int64_t)po.tasks[key].size();
+    // The mixed kernel takes any task: where the mixed tasks and the others of their rows per lane are fewer than the warp
+    // slots, they go together, one bucket less to launch against its 4 % on the others.
+    auto bucket_of = [&](int key) {
+        if (bucket_mixed(key) || bucket_rows(key) < 2) return key;
+        const int64_t mixed = key_count[(size_t)key + kBucketMixed];
+        return mixed > 0 && mixed + key_count[(size_t)key] <= (int64_t)ctx->sm_count * 12 ? key + kBucketMixed : key;
+    };
+    std::vector<int64_t> bucket_count(kNumBucketKeys, 0);
+    for (int key = 0; key < kNumBucketKeys; key++) bucket_count[(size_t)bucket_of(key)] += key_count[(size_t)key];
+    std::partial_sum(bucket_count.begin(), bucket_count.end(), bucket_pos.begin() + 1);
     for (auto &po : parts) {
         max_multi_cols = std::max(max_multi_cols, po.max_multi_cols);
         n_direct += (int64_t)po.direct.size();
@@ -439,10 +454,11 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
         std::vector<const F32Task *> src_task;
         src_task.reserve((size_t)n);
         for (auto &po : parts)
-            for (size_t i = 0; i < po.tasks[key].size(); i++) {
-                order.emplace_back(-po.cost[key][i], (int64_t)src_task.size());
-                src_task.push_back(&po.tasks[key][i]);
-            }
+            for (int from = 0; from < kNumBucketKeys; from++)
+                for (size_t i = 0; i < po.tasks[from].size() && bucket_of(from) == (int)key; i++) {
+                    order.emplace_back(-po.cost[from][i], (int64_t)src_task.size());
+                    src_task.push_back(&po.tasks[from][i]);
+                }
         std::sort(order.begin(), order.end());
         F32Task *dst = b.h_tasks.p + bucket_pos[(size_t)key];
         for (int64_t i = 0; i < n; i++) dst[i] = *src_task[(size_t)order[(size_t)i].second];
@@ -457,10 +473,13 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
         b.buckets.push_back(Bucket{key, (int)bucket_pos[(size_t)key], (int)n, grid, 0});
     }
     // most rows first (their tasks are the longest); each multi-strip bucket its own part of the strip scratch
-    std::reverse(b.buckets.begin(), b.buckets.end());
+    std::sort(b.buckets.begin(), b.buckets.end(), [](const Bucket &x, const Bucket &y) {
+        const int mx = x.key & kBucketMulti, my = y.key & kBucketMulti;
+        return mx != my ? mx > my : bucket_rows(x.key) != bucket_rows(y.key) ? bucket_rows(x.key) > bucket_rows(y.key) : x.key > y.key;
+    });
     b.scratch32_blocks = 0;
     for (auto &bk : b.buckets)
-        if (bk.key & 16) {
+        if (bk.key & kBucketMulti) {
             bk.scratch_block = b.scratch32_blocks;
             b.scratch32_blocks += bk.grid;
         }
@@ -694,7 +713,7 @@ int fork_buckets(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s,
             GHMM_CUDA(cudaStreamWaitEvent(st, ctx->fork_ev[kForkStreams], 0), "fork");
         const Bucket &bk = b.buckets[(size_t)i];
         DevBatch d = b.dev;
-        if (bk.key & 16) d.scratch32 += (int64_t)bk.scratch_block * kWarpsPerBlock * d.scratch32_cols * 3;
+        if (bk.key & kBucketMulti) d.scratch32 += (int64_t)bk.scratch_block * kWarpsPerBlock * d.scratch32_cols * 3;
         rc = launch(bk, d, st);
     }
     for (int lane = 1; lane < lanes; lane++) {

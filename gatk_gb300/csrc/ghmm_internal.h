@@ -14,7 +14,18 @@ constexpr uint8_t kColFirst = 0x40;
 constexpr uint8_t kColLast = 0x80;
 constexpr int kMaxK32 = 8;      // FP32 kernel: rows per lane (strip = 32*K rows)
 constexpr int kMaxReadLen = 1 << 20;
-constexpr int kNumBucketKeys = 32;       // bucket key = rows per lane (1..8) | 16 for multi-strip
+// Bucket key: rows per lane (2..8), + kBucketMixed for tasks of mixed haplotypes, + kBucketMulti for tasks of several
+// strips.  Mixed: some haplotype has fewer than kShortHapCols columns, of which the first lane ends before the last lane
+// has started it, so that the kernel has to look for such events step by step; and more than a quarter of the columns lie
+// that far behind a longer haplotype's start, where it need not.  The other tasks with short haplotypes are checked at
+// every step.  (FP32 pass, 24 haplotypes of 400 columns and one of 62 a task: every step checked 18.6 ms, mixed 13.1, with
+// one of 63 instead 12.6; haplotypes of 50 columns alone: checked 5.22, mixed 5.27; 50 and 70 in turn: 6.10 and 6.01.)
+constexpr int kNumBucketKeys = 32;
+constexpr int kBucketMixed = 7;
+constexpr int kBucketMulti = 16;
+constexpr bool bucket_mixed(int key) { return (key & 15) > kMaxK32; }
+constexpr int bucket_rows(int key) { return (key & 15) - (bucket_mixed(key) ? kBucketMixed : 0); }
+constexpr int kShortHapCols = 63;
 constexpr int kCounterBucketBase = 8;    // counters[8 + key]: bucket task cursors
 constexpr int kNumCounters = 64;
 constexpr int kMaxHapLen = 1 << 20;
@@ -101,7 +112,7 @@ constexpr int kCodePad = 64;
 // worst case, and a pair whose rescaled states do overflow sums to a non-finite value and moves to the exact tier, so
 // this only keeps pairs that would almost surely overflow from running twice).
 constexpr double kMaxGrowth64 = 1e15;
-int fp32_kernel_occupancy(int k, int block, int *blocks_per_sm);
+int fp32_kernel_occupancy(int key, int block, int *blocks_per_sm);
 int fp64_kernel_occupancy(int *blocks_per_sm);
 
 // PD-HMM (pd.cu): per haplotype column, the PD flag byte (PartiallyDeterminedHaplotype bits) and the HMM state

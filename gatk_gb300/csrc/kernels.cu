@@ -87,9 +87,11 @@ struct Fp32MinBlocks {
 
 // The bucket's task range and cursor live in device memory (B.bucket_info, B.counters), so the launch
 // arguments do not depend on the batch and a captured CUDA graph can be replayed for every batch.
-template <int K, bool MULTI>
+// MIXED: tasks of short and long haplotypes (kBucketMixed).  A kernel of its own, since the loops of a third form in one
+// kernel make the compiler's code for the other two up to 4 % slower.
+template <int K, bool MULTI, bool MIXED>
 __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kernel(DevTables T, DevBatch B) {
-    constexpr int KEY = K | (MULTI ? 16 : 0);
+    constexpr int KEY = K + (MIXED ? kBucketMixed : 0) + (MULTI ? kBucketMulti : 0);
     const int task_begin = B.bucket_info[KEY], task_count = B.bucket_info[kNumBucketKeys + KEY];
     const int counter_slot = kCounterBucketBase + KEY;
     constexpr int S = 32 * K;
@@ -138,9 +140,11 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
         const uint8_t *stream = B.hap_code + col0;
         const int nstrips = MULTI ? task.nstrips : 1;
         bool long_haps = true;
-        for (int h = task.hap_begin + lane; h < task.hap_end; h += 32)
-            long_haps &= B.hap_off[h + 1] - B.hap_off[h] >= 63;
-        long_haps = __all_sync(kFull, long_haps);
+        if constexpr (!MIXED) {
+            for (int h = task.hap_begin + lane; h < task.hap_end; h += 32)
+                long_haps &= B.hap_off[h + 1] - B.hap_off[h] >= kShortHapCols;
+            long_haps = __all_sync(kFull, long_haps);
+        }
 
         for (int strip = 0; strip < nstrips; ++strip) {
             float2 cb[K], cc[K], ce[K], cdd[K];
@@ -326,7 +330,73 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
             using Reset = std::integral_constant<int, kReset>;
             using Zero = std::integral_constant<int, kZero>;
             int s = 0;
-            if (long_haps) {
+            if constexpr (MIXED) {
+                // as below for the haplotypes of 63 columns or more; from the boundary of a shorter one on, events of several
+                // boundaries overlap, and the steps are checked until those of the next long haplotype's are over
+                const int dummies = max(task.pad_a, rb >= 0 ? task.pad_b : 0) - strip * S;  // on top of this strip
+                const int n_reset = dummies >= 0 ? min(30, dummies / K + 1) : 0;  // lanes with or right below dummy rows
+                bool last_long = false;
+                for (int j = 0; j < nh_task;) {  // s: haplotype j's first column
+                    int end = (int)(hoff[j + 1] - col0);
+                    last_long = end - s >= kShortHapCols;
+                    if (last_long) {
+                        const float init = __ldg(B.hap_init_f + task.hap_begin + j);
+                        int l = 0;
+#pragma unroll 1
+                        for (; l < n_reset; ++l, s += 2) {
+                            refill(s);
+                            step(s, Reset{}, l, init);
+                            refill(s + 1);
+                            step(s + 1, Plain{}, 0, 0.f);
+                        }
+#pragma unroll 1
+                        for (; l < 30; ++l, s += 2) {
+                            refill(s);
+                            step(s, Zero{}, l, 0.f);
+                            refill(s + 1);
+                            step(s + 1, Plain{}, 0, 0.f);
+                        }
+                        refill(s);
+                        step(s, Reset{}, 30, init);
+                        refill(s + 1);
+                        step(s + 1, Plain{}, 0, 0.f);
+                        if (j > 0 && last_strip && lane == 31) emit(task.hap_begin + j - 1);
+                        refill(s + 2);
+                        step(s + 2, Reset{}, 31, init);
+                        s += 3;
+                        ++j;
+                    } else {
+                        hap = task.hap_begin + j - 1;
+                        int stop = nsteps;
+                        for (int begin = s; ++j < nh_task;) {  // haplotype j - 1, from column begin to end, is short
+                            begin = end;
+                            end = (int)(hoff[j + 1] - col0);
+                            if (end - begin >= kShortHapCols) {
+                                stop = begin + kShortHapCols;
+                                last_long = true;
+                                ++j;
+                                break;
+                            }
+                        }
+#pragma unroll 2
+                        for (; s < stop; ++s) {
+                            refill(s);
+                            step(s, std::integral_constant<int, kCheck>{}, 0, 0.f);
+                        }
+                    }
+                    const int until = j < nh_task ? end : nsteps;
+                    while (s < until) {
+                        refill(s);
+                        const int stop = MULTI && strip > 0 ? min(until, (s | 31) + 1) : until;
+                        // unrolled: the scheduler interleaves one step's I~ chain and shuffles with the following steps' M~
+                        // and D~ (16 measured best of 2-32; with the strip boundary 8 of 4, 8 and 16)
+                        constexpr int kUnroll = MULTI ? 8 : 16;
+#pragma unroll kUnroll
+                        for (; s < stop; ++s) step(s, Plain{}, 0, 0.f);
+                    }
+                }
+                if (last_long && last_strip && lane == 31) emit(task.hap_end - 1);
+            } else if (long_haps) {
                 // Haplotypes of 63 columns or more: at a boundary at column hb, lane l starts the next haplotype at step
                 // hb + 2 l and lane 31 ends the previous one at step hb + 61, so which steps have events, and for which
                 // lane, is known without looking at a column code, and every other step between two starts is plain.
@@ -373,7 +443,7 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
                     s += 3;
                 }
                 if (last_strip && lane == 31) emit(task.hap_end - 1);
-            } else {
+            } else {  // most are shorter
 #pragma unroll 2
                 for (; s < nsteps; ++s) {
                     refill(s);
@@ -560,26 +630,29 @@ static size_t fp32_smem_bytes(int k, int block, bool multi) {
     return (size_t)(block / 32) * (((k + 1) / 2) * kBases * 32 + (multi ? 64 : 0)) * sizeof(float4);
 }
 
-template <int K, bool MULTI>
+template <int K, bool MULTI, bool MIXED>
 static int launch_fp32_k(const DevTables &t, const DevBatch &b, int grid, int block, cudaStream_t s) {
     const size_t smem = fp32_smem_bytes(K, block, MULTI);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(fp32_bucket_kernel<K, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(fp32_bucket_kernel<K, MULTI, MIXED>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    fp32_bucket_kernel<K, MULTI><<<grid, block, smem, s>>>(t, b);
+    fp32_bucket_kernel<K, MULTI, MIXED><<<grid, block, smem, s>>>(t, b);
     return (int)cudaGetLastError();
 }
 
-int launch_fp32_bucket(const DevTables &t, const DevBatch &b, int k, int grid, int block, cudaStream_t s) {
-    // k encodes rows per lane in the low 4 bits and the multi-strip flag in bit 4
-    const bool multi = (k & 16) != 0;
-    switch (k & 15) {
-#define GHMM_CASE(KK)                                                                                   \
-    case KK:                                                                                            \
-        return multi ? launch_fp32_k<KK, true>(t, b, grid, block, s) : launch_fp32_k<KK, false>(t, b, grid, block, s);
-        GHMM_CASE(1)
+// f(rows per lane, several strips, mixed haplotypes), as integral constants, of a bucket key
+template <typename F>
+static int with_bucket(int key, F f) {
+    switch (bucket_rows(key)) {
+#define GHMM_CASE(KK)                                                                                                     \
+    case KK: {                                                                                                            \
+        using K = std::integral_constant<int, KK>;                                                                        \
+        if (key & kBucketMulti)                                                                                           \
+            return bucket_mixed(key) ? f(K{}, std::true_type{}, std::true_type{}) : f(K{}, std::true_type{}, std::false_type{}); \
+        return bucket_mixed(key) ? f(K{}, std::false_type{}, std::true_type{}) : f(K{}, std::false_type{}, std::false_type{}); \
+    }
         GHMM_CASE(2)
         GHMM_CASE(3)
         GHMM_CASE(4)
@@ -593,30 +666,18 @@ int launch_fp32_bucket(const DevTables &t, const DevBatch &b, int k, int grid, i
     }
 }
 
-int fp32_kernel_occupancy(int k, int block, int *blocks_per_sm) {
-    const bool multi = (k & 16) != 0;
-    cudaError_t e = cudaErrorInvalidValue;
-    switch (k & 15) {
-#define GHMM_OCC(KK)                                                                                              \
-    case KK:                                                                                                      \
-        e = multi ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fp32_bucket_kernel<KK, true>, block,  \
-                                                                  fp32_smem_bytes(KK, block, true))                          \
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fp32_bucket_kernel<KK, false>, block, \
-                                                                  fp32_smem_bytes(KK, block, false));                         \
-        break;
-        GHMM_OCC(1)
-        GHMM_OCC(2)
-        GHMM_OCC(3)
-        GHMM_OCC(4)
-        GHMM_OCC(5)
-        GHMM_OCC(6)
-        GHMM_OCC(7)
-        GHMM_OCC(8)
-#undef GHMM_OCC
-        default:
-            break;
-    }
-    return (int)e;
+int launch_fp32_bucket(const DevTables &t, const DevBatch &b, int key, int grid, int block, cudaStream_t s) {
+    return with_bucket(key, [&](auto k, auto multi, auto mixed) {
+        return launch_fp32_k<k.value, multi.value, mixed.value>(t, b, grid, block, s);
+    });
+}
+
+int fp32_kernel_occupancy(int key, int block, int *blocks_per_sm) {
+    return with_bucket(key, [&](auto k, auto multi, auto mixed) {
+        return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            blocks_per_sm, fp32_bucket_kernel<k.value, multi.value, mixed.value>, block,
+            fp32_smem_bytes(k.value, block, multi.value));
+    });
 }
 
 int launch_read_scale(const DevTables &t, const DevBatch &b, int64_t n_reads, float2 *scale, int sm_count,

@@ -33,7 +33,7 @@ constexpr int kWarpsPerBlock = kBlock / 32;
 constexpr int kRouteFp64Log10 = -100;
 
 struct Bucket {
-    int key;  // rows-per-lane | 16 if multi-strip
+    int key;  // ghmm_internal.h
     int begin, count;
     int grid;
     int scratch_block;  // multi-strip buckets run side by side: first block of this bucket's part of the strip scratch
