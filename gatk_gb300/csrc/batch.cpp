@@ -299,7 +299,8 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
         std::vector<F32Task> tasks[kNumBucketKeys];
         std::vector<int64_t> cost[kNumBucketKeys];
         std::vector<PairRef> direct, direct_exact;
-        int64_t max_multi_cols = 0, cells_direct = 0;
+        int64_t max_cols[kNumBucketKeys]{};  // of the buckets of several strips: the longest task's columns
+        int64_t cells_direct = 0;
     };
     const int64_t n_parts = std::max<int64_t>(1, std::min<int64_t>(G, (int64_t)threads * 4));
     std::vector<PartOut> parts((size_t)n_parts);
@@ -413,7 +414,7 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
                     t.pad_a = nstrips * S - Ra - kAccRows;
                     t.pad_b = rb >= 0 ? nstrips * S - Rb - kAccRows : nstrips * S;
                     const int task_key = key + (ch.mixed ? kBucketMixed : 0);
-                    if (multi) po.max_multi_cols = std::max(po.max_multi_cols, ch.cols);
+                    if (multi) po.max_cols[task_key] = std::max(po.max_cols[task_key], ch.cols);
                     po.tasks[task_key].push_back(t);
                     po.cost[task_key].push_back((ch.cols + 31) * K * nstrips);
                 }
@@ -422,7 +423,7 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
     }, 1);
     // buckets in key order, each ordered longest task first (ties keep region order)
     b.buckets.clear();
-    int64_t total_tasks = 0, max_multi_cols = 0, n_direct = 0, n_direct_exact = 0;
+    int64_t total_tasks = 0, n_direct = 0, n_direct_exact = 0;
     b.cells_direct = 0;
     std::vector<int64_t> bucket_pos(kNumBucketKeys + 1, 0);
     std::vector<int64_t> key_count(kNumBucketKeys, 0);
@@ -439,7 +440,6 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
     for (int key = 0; key < kNumBucketKeys; key++) bucket_count[(size_t)bucket_of(key)] += key_count[(size_t)key];
     std::partial_sum(bucket_count.begin(), bucket_count.end(), bucket_pos.begin() + 1);
     for (auto &po : parts) {
-        max_multi_cols = std::max(max_multi_cols, po.max_multi_cols);
         n_direct += (int64_t)po.direct.size();
         n_direct_exact += (int64_t)po.direct_exact.size();
         b.cells_direct += po.cells_direct;
@@ -470,18 +470,22 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
         if (fp32_kernel_occupancy(key, kBlock, &bpsm) != 0 || bpsm <= 0) bpsm = 1;
         const int64_t want = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * bpsm));
-        b.buckets.push_back(Bucket{key, (int)bucket_pos[(size_t)key], (int)n, grid, 0});
+        int64_t cols = 0;
+        for (int from = 0; from < kNumBucketKeys; from++)
+            if (bucket_of(from) == key)
+                for (auto &po : parts) cols = std::max(cols, po.max_cols[from]);
+        b.buckets.push_back(Bucket{key, (int)bucket_pos[(size_t)key], (int)n, grid, 0, cols});
     }
     // most rows first (their tasks are the longest); each multi-strip bucket its own part of the strip scratch
     std::sort(b.buckets.begin(), b.buckets.end(), [](const Bucket &x, const Bucket &y) {
         const int mx = x.key & kBucketMulti, my = y.key & kBucketMulti;
         return mx != my ? mx > my : bucket_rows(x.key) != bucket_rows(y.key) ? bucket_rows(x.key) > bucket_rows(y.key) : x.key > y.key;
     });
-    b.scratch32_blocks = 0;
+    b.scratch32_size = 0;
     for (auto &bk : b.buckets)
         if (bk.key & kBucketMulti) {
-            bk.scratch_block = b.scratch32_blocks;
-            b.scratch32_blocks += bk.grid;
+            bk.scratch_begin = b.scratch32_size;
+            b.scratch32_size += (int64_t)bk.grid * kWarpsPerBlock * bk.scratch_cols;
         }
     b.n_tasks = total_tasks;
     b.n_direct = n_direct;
@@ -499,7 +503,6 @@ int batch_marshal(ghmm_ctx *ctx, const Source &src, ghmm_batch &b) {
             k += (int64_t)po.direct_exact.size();
         }
     }
-    b.scratch32_cols = max_multi_cols;
     int bpsm64 = 0;
     if (fp64_kernel_occupancy(&bpsm64) != 0 || bpsm64 <= 0) bpsm64 = 1;
     b.fp64_grid = ctx->sm_count * bpsm64;
@@ -528,8 +531,7 @@ int batch_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s) {
     GHMM_CUDA(b.d_out.reserve((size_t)std::max<int64_t>(b.n_out, 1)), "device output");
     GHMM_CUDA(b.d_counters.reserve(kNumCounters + 2 * kNumBucketKeys), "device counters");
     GHMM_CUDA(b.d_nout.reserve(1), "device output count");
-    const size_t s32 = (size_t)b.scratch32_blocks * kWarpsPerBlock * (size_t)b.scratch32_cols * 3;
-    GHMM_CUDA(b.d_scratch32.reserve(std::max<size_t>(s32, 1)), "device FP32 strip scratch");
+    GHMM_CUDA(b.d_scratch32.reserve((size_t)std::max<int64_t>(b.scratch32_size, 1)), "device FP32 strip scratch");
     // columns of the FP64 strip scratch per warp: a haplotype, or a run of them (runs end at what fits)
     const bool runs64 = b.max_hap_len <= kFp64RunCols && b.max_read_len < kFp64SplitRows;
     const int64_t cols64 = (int64_t)std::max(b.max_hap_len, 1) * (runs64 ? kFp64Run : 1);
@@ -577,7 +579,7 @@ int batch_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s) {
     d.rerun_capacity = capacity;
     d.force_rerun_every = ctx->debug_force_rerun;
     d.scratch32 = b.d_scratch32.p;
-    d.scratch32_cols = b.scratch32_cols;
+    d.scratch32_cols = 0;
     d.scratch64 = b.d_scratch64.p;
     d.scratch64_cols = cols64;
     d.read_scale = b.d_read_scale.p;
@@ -713,7 +715,10 @@ int fork_buckets(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s,
             GHMM_CUDA(cudaStreamWaitEvent(st, ctx->fork_ev[kForkStreams], 0), "fork");
         const Bucket &bk = b.buckets[(size_t)i];
         DevBatch d = b.dev;
-        if (bk.key & kBucketMulti) d.scratch32 += (int64_t)bk.scratch_block * kWarpsPerBlock * d.scratch32_cols * 3;
+        if (bk.key & kBucketMulti) {
+            d.scratch32 += bk.scratch_begin;
+            d.scratch32_cols = bk.scratch_cols;
+        }
         rc = launch(bk, d, st);
     }
     for (int lane = 1; lane < lanes; lane++) {
@@ -780,7 +785,7 @@ int batch_enqueue(ghmm_ctx *ctx, ghmm_batch &b, int mode, cudaStream_t s) {
     const int fp64_args[2] = {b.max_read_len >= kFp64SplitRows, b.fp64_grid};
     sig.insert(sig.end(), (const unsigned char *)fp64_args, (const unsigned char *)fp64_args + sizeof(fp64_args));
     for (auto &bk : b.buckets) {
-        const int kg[2] = {bk.key, bk.grid};
+        const int64_t kg[4] = {bk.key, bk.grid, bk.scratch_begin, bk.scratch_cols};
         const unsigned char *k = (const unsigned char *)kg;
         sig.insert(sig.end(), k, k + sizeof(kg));
     }

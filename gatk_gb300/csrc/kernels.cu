@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128, Fp32MinBlocks<K>::value) fp32_bucket_kern
     // (FP32 pass of reads of 510 bases x haplotypes of 600: 3,110 GCUPS, with the ring 3,845).
     float4 *scratch = nullptr, *ring = nullptr;
     if (MULTI) {
-        scratch = reinterpret_cast<float4 *>(B.scratch32) + warp_global * B.scratch32_cols;
+        scratch = B.scratch32 + warp_global * B.scratch32_cols;
         ring = prior_smem4 + 4 * (KP * kBases * 32) + (threadIdx.x >> 5) * 64;
     }
 

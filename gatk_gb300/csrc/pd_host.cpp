@@ -292,7 +292,7 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s) 
         memcpy(sig.data(), &b.dev, sizeof(DevBatch));
         memcpy(sig.data() + sizeof(DevBatch), &b.pd, sizeof(PdPlanes));
         for (auto &bk : b.buckets) {
-            const int kg[3] = {bk.key, bk.grid, bk.count};
+            const int64_t kg[5] = {bk.key, bk.grid, bk.count, bk.scratch_begin, bk.scratch_cols};
             const unsigned char *k3 = (const unsigned char *)kg;
             sig.insert(sig.end(), k3, k3 + sizeof(kg));
         }
@@ -307,7 +307,7 @@ int pd_forward_enqueue(ghmm_ctx *ctx, ghmm_batch &b, bool fp32, cudaStream_t s) 
                     if (pd_bucket_occupancy(bk.key, &bp) != 0 || bp <= 0) bp = 1;
                     const int64_t want = (bk.count + kWarpsPerBlock - 1) / kWarpsPerBlock;
                     int g = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->sm_count * bp));
-                    if (bk.key & 16) g = std::min(g, bk.grid);  // the strip scratch is sized for the regular kernel's grid
+                    if (bk.key & kBucketMulti) g = std::min(g, bk.grid);  // the strip scratch is sized for the regular kernel's grid
                     const int e = launch_pd_bucket(ctx->tables, d, b.pd, bk.key, g, st);
                     return e ? cuda_fail(ctx, (cudaError_t)e, "PD-HMM packed launch") : GHMM_OK;
                 });

@@ -125,7 +125,9 @@ __global__ void __launch_bounds__(128, PdMinBlocks<K>::value) pd_bucket_kernel(D
     // strip boundary of multi-strip tasks: per column lane 31's hand-over (I~ and the M~ inner sum) for lane 0 of
     // the next strip, as the regular kernel passes it
     float2 *scratch = nullptr;
-    if (MULTI) scratch = B.scratch32 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * B.scratch32_cols * 3;
+    if (MULTI)
+        scratch = reinterpret_cast<float2 *>(B.scratch32 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) *
+                                                               B.scratch32_cols);
 
     for (;;) {
         int t = 0;

@@ -36,7 +36,9 @@ struct Bucket {
     int key;  // ghmm_internal.h
     int begin, count;
     int grid;
-    int scratch_block;  // multi-strip buckets run side by side: first block of this bucket's part of the strip scratch
+    // buckets of several strips run side by side: where this bucket's part of the strip scratch begins, and its columns a
+    // warp (its longest task's)
+    int64_t scratch_begin, scratch_cols;
 };
 // The most kernels of one forward that run side by side: the caller's stream and kForkStreams forked from it.
 constexpr int kForkStreams = 4;
@@ -102,7 +104,7 @@ struct ghmm_batch {
     DevBuf<uint8_t> d_pd;
     bool has_pd = false;
     PdPlanes pd{};
-    DevBuf<float2> d_scratch32;
+    DevBuf<float4> d_scratch32;
     DevBuf<double> d_scratch64;
     DevBuf<float2> d_read_scale;  // per read: the FP32 pass's log2 a_R as (2^-(la - n), n), from launch_read_scale
     // sizes
@@ -117,8 +119,7 @@ struct ghmm_batch {
     double ms_host_copy = 0, ms_host_tasks = 0;  // host time of the last marshal: copy + checks, task building
     int64_t n_direct_fp64mode = 0, n_fp64mode_exact = 0;
     std::vector<uint8_t> read_exact;  // reads whose pairs go to the exact FP64 tier directly
-    int64_t scratch32_cols = 0;
-    int scratch32_blocks = 0;
+    int64_t scratch32_size = 0;  // of all buckets
     int fp64_grid = 0;
     // last forward
     int last_mode = -1;
