@@ -16,7 +16,7 @@
 // the backward runs the strips last to first, and the adjoint values a strip's first row hands the row above are
 // kept in scratch per column for the strip above it.
 //  * Forward: the whole warp front (each lane's K rows of M, I, D plus the diagonal inputs) is saved to scratch
-//    every kSeg (8) steps (the checkpoints); lane 31 sums the last row into L_s (scaled likelihood).
+//    every SEG (8 or 16) steps (the checkpoints); lane 31 sums the last row into L_s (scaled likelihood).
 //  * Backward: segments are processed last to first.  Each segment's forward is recomputed from its checkpoint,
 //    keeping every step's front, and then the adjoint wavefront runs over it in reverse: lane l at reverse step s
 //    handles column s - l, receiving from lane l+1 (the row below) by __shfl_down_sync.  Adjoints are seeded with
@@ -45,7 +45,8 @@ constexpr unsigned kFullMask = 0xffffffffu;
 // then nearly fit its L1, and the checkpoints (2.5 KB a segment and warp) stay a minor stream.  Backward of 4,096 pairs
 // of 150 x 300 bases: 855 us at 16, 810 at 8, 815 at 6, 855 at 4; of 8,345 pairs of up to 250 x 600: 3,113, 2,994,
 // 3,058, 3,149 (both at 16 with fronts of single values and each loaded twice: 854 and 3,588).
-constexpr int kSeg = 8;
+// Pairs so long that a full grid's checkpoints would exceed the scratch budget run at 16 (calib_seg).
+constexpr int kSeg = 8, kSegLong = 16;
 constexpr int kCalibBlock = 64;
 
 template <typename T>
@@ -190,7 +191,7 @@ struct Vec16<double> {
 template <typename T, int K>
 constexpr int kFrontSize = (3 * K + 3 + Vec16<T>::n - 1) / Vec16<T>::n * Vec16<T>::n;  // values a lane, whole vectors
 
-// scratch layout per warp (all T): checkpoints [nck][front][32], segment fronts [kSeg][front][32], the strips' last
+// scratch layout per warp (all T): checkpoints [nck][front][32], segment fronts [segment's steps][front][32], the strips' last
 // rows [nstrips - 1][H][3] (forward), and two buffers [H][4] of first-row adjoint values (backward, by strip parity)
 template <typename T, int K>
 __device__ __forceinline__ void save_front(T *dst, const Front<T, K> &f, int lane) {
@@ -244,7 +245,7 @@ __device__ __forceinline__ void load_front(const T *src, Front<T, K> &f, int lan
 
 // MULTI: reads may need more than one strip (K = 8 batches with reads longer than 256 bases); otherwise every read fits
 // one strip and the strip logic folds away.
-template <typename T, int K, bool BACKWARD, bool MULTI>
+template <typename T, int K, bool BACKWARD, bool MULTI, int SEG>
 __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int64_t pair, T *scratch, double *loglik,
                            const double *weights, float *grad_open, float *grad_cont, int *need_fp64, bool fp64_pass) {
     constexpr int F = kFrontSize<T, K>;  // values per lane in a front
@@ -264,9 +265,9 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
     const uint8_t *hb = in.hap_bases + hoff;
     const T init = CalibScale<T>::init(H);
     const int nsteps = H + 31;
-    const int nseg = (nsteps + kSeg - 1) / kSeg;
+    const int nseg = BACKWARD ? (nsteps + SEG - 1) / SEG : 0;
     T *seg = scratch + (size_t)nseg * F * 32;
-    T *fwd_bnd = seg + (size_t)kSeg * F * 32;                 // [nstrips - 1][H][3]
+    T *fwd_bnd = seg + (BACKWARD ? (size_t)SEG * F * 32 : 0);  // [nstrips - 1][H][3]
     T *adj_bnd = fwd_bnd + (size_t)(nstrips - 1) * H * 3;     // [2][H][4]
     Rows<T, K> w;
     Front<T, K> f;
@@ -281,7 +282,7 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
         for (int k = 0; k < K; ++k) f.M[k] = f.I[k] = f.D[k] = (T)0;
         f.gM = f.gI = f.gD = (T)0;
         for (int s = 0; s < nsteps; ++s) {
-            if (BACKWARD && s % kSeg == 0) save_front<T, K>(scratch + (size_t)(s / kSeg) * F * 32, f, lane);
+            if (BACKWARD && s % SEG == 0) save_front<T, K>(scratch + (size_t)(s / SEG) * F * 32, f, lane);
             T uM, uI, uD;
             fwd_step<T, K>(w, f, hb, H, s, lane, pad, init, bnd, uM, uI, uD);
             const int c = s - lane;
@@ -321,7 +322,7 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
             for (int k = 0; k < K; ++k) f.M[k] = f.I[k] = f.D[k] = (T)0;
             f.gM = f.gI = f.gD = (T)0;
             for (int s = 0; s < nsteps; ++s) {
-                if (s % kSeg == 0) save_front<T, K>(scratch + (size_t)(s / kSeg) * F * 32, f, lane);
+                if (s % SEG == 0) save_front<T, K>(scratch + (size_t)(s / SEG) * F * 32, f, lane);
                 T uM, uI, uD;
                 fwd_step<T, K>(w, f, hb, H, s, lane, pad, init, bnd, uM, uI, uD);
             }
@@ -340,7 +341,7 @@ __device__ void calib_pair(const DevTables &TB, const ghmm_calib_batch &in, int6
         const bool below = lane != 31 || !last;  // lane 31 of the last strip holds the read's last row
         Front<T, K> cur;  // the front after the step being reversed
         for (int sg = nseg - 1; sg >= 0; --sg) {
-            const int s0 = sg * kSeg, s1 = min(s0 + kSeg, nsteps);
+            const int s0 = sg * SEG, s1 = min(s0 + SEG, nsteps);
             // recompute the segment's fronts (front after each step, plus the step's "up" values)
             Front<T, K> r;
             load_front<T, K>(scratch + (size_t)sg * F * 32, r, lane);
@@ -470,7 +471,7 @@ struct CalibMinBlocks {
     static constexpr int value = sizeof(T) == 4 && BACKWARD && K <= 5 ? 6 : 0;
 };
 
-template <typename T, int K, bool BACKWARD, bool MULTI>
+template <typename T, int K, bool BACKWARD, bool MULTI, int SEG>
 __global__ void __launch_bounds__(kCalibBlock, CalibMinBlocks<T, K, BACKWARD>::value) calib_kernel(DevTables TB, ghmm_calib_batch in, T *scratch,
                                                             int64_t scratch_per_warp, double *loglik,
                                                             const double *weights, float *grad_open, float *grad_cont,
@@ -480,8 +481,8 @@ __global__ void __launch_bounds__(kCalibBlock, CalibMinBlocks<T, K, BACKWARD>::v
     T *my = scratch + warp * scratch_per_warp;
     for (int64_t p = warp; p < in.n_pairs; p += nwarps) {
         if (fp64_pass && !need_fp64[p]) continue;
-        calib_pair<T, K, BACKWARD, MULTI>(TB, in, p, my, loglik, weights, grad_open, grad_cont, need_fp64,
-                                          fp64_pass != 0);
+        calib_pair<T, K, BACKWARD, MULTI, SEG>(TB, in, p, my, loglik, weights, grad_open, grad_cont, need_fp64,
+                                               fp64_pass != 0);
         __syncwarp();
     }
 }
@@ -544,12 +545,12 @@ __global__ void __launch_bounds__(256) calib_fold_kernel(const int64_t *index, i
 }
 
 // Blocks of one instantiation resident on an SM (from its registers), looked up once per process.
-template <typename T, int K, bool BACKWARD, bool MULTI>
+template <typename T, int K, bool BACKWARD, bool MULTI, int SEG>
 int calib_resident_blocks() {
     static std::atomic<int> blocks{0};
     int b = blocks.load(std::memory_order_relaxed);
     if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, calib_kernel<T, K, BACKWARD, MULTI>, kCalibBlock, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, calib_kernel<T, K, BACKWARD, MULTI, SEG>, kCalibBlock, 0) !=
                 cudaSuccess ||
             b < 1)
             b = 1;
@@ -560,10 +561,10 @@ int calib_resident_blocks() {
 
 }  // namespace
 
-int64_t calib_scratch_per_warp(int k, int max_hap_len, int max_read_len, bool fp64) {
+int64_t calib_scratch_per_warp(int k, int max_hap_len, int max_read_len, bool fp64, int seg) {
     const int64_t vec = fp64 ? 2 : 4, F = (3 * k + 3 + vec - 1) / vec * vec;
     const int64_t nsteps = max_hap_len + 31;
-    const int64_t fronts = (nsteps + kSeg - 1) / kSeg + kSeg;
+    const int64_t fronts = (nsteps + seg - 1) / seg + seg;
     const int64_t nstrips = ((int64_t)max_read_len + 32 * k - 1) / (32 * k);
     const int64_t boundaries = (nstrips - 1) * max_hap_len * 3 + 2 * (int64_t)max_hap_len * 4;
     return (fronts * F * 32 + boundaries + 3) / 4 * 4 * (fp64 ? 8 : 4);  // whole 16-byte vectors
@@ -576,25 +577,54 @@ int64_t calib_scratch_per_warp(int k, int max_hap_len, int max_read_len, bool fp
 int calib_grid(int sm_count) { return sm_count * 6; }
 int calib_block() { return kCalibBlock; }
 
+// Steps between checkpoints for a call's largest sizes: eight, unless their scratch within the budget
+// holds fewer warps than the FP32 backward keeps resident (from haplotypes of some 4,000 columns on at the default 4 GiB).
+// Backward of 2,432 pairs, eight and sixteen: 150 x 5,000 bases 8.8 and 8.2 ms, 150 x 8,000 16.5 and 12.8, 250 x 4,500 11.4
+// and 9.2, 250 x 7,000 21.8 and 17.3; of 1,216 of 600 x 4,500 33.0 and 19.7.
+int calib_seg(int k, int max_hap_len, int max_read_len, int64_t budget, int sm_count) {
+    int resident = 1;
+    switch (k) {
+#define GHMM_CALIB_RESIDENT(KK) \
+    case KK: resident = calib_resident_blocks<float, KK, true, false, kSeg>(); break;
+        GHMM_CALIB_RESIDENT(1)
+        GHMM_CALIB_RESIDENT(2)
+        GHMM_CALIB_RESIDENT(3)
+        GHMM_CALIB_RESIDENT(4)
+        GHMM_CALIB_RESIDENT(5)
+        GHMM_CALIB_RESIDENT(6)
+        GHMM_CALIB_RESIDENT(7)
+#undef GHMM_CALIB_RESIDENT
+        default:
+            resident = max_read_len > 32 * 8 ? calib_resident_blocks<float, 8, true, true, kSeg>()
+                                             : calib_resident_blocks<float, 8, true, false, kSeg>();
+    }
+    const int64_t warps = (int64_t)std::min(calib_grid(sm_count), sm_count * resident) * (kCalibBlock / 32);
+    return calib_scratch_per_warp(k, max_hap_len, max_read_len, true, kSeg) * warps <= budget ? kSeg : kSegLong;
+}
+
 int launch_calib(const DevTables &TB, const ghmm_calib_batch &in, int k, bool backward, bool fp64, void *scratch,
                  int64_t scratch_bytes_per_warp, double *loglik, const double *weights, float *grad_open,
-                 float *grad_cont, int *need_fp64, int grid, int sm_count, cudaStream_t s) {
-#define GHMM_CALIB_ONE(T, KK, BWD, MUL)                                                                             \
-    calib_kernel<T, KK, BWD, MUL>                                                                                   \
-        <<<std::min(grid, sm_count * calib_resident_blocks<T, KK, BWD, MUL>()), kCalibBlock, 0, s>>>(              \
+                 float *grad_cont, int *need_fp64, int seg, int grid, int sm_count, cudaStream_t s) {
+#define GHMM_CALIB_ONE(T, KK, BWD, MUL, SEG)                                                                        \
+    calib_kernel<T, KK, BWD, MUL, SEG>                                                                              \
+        <<<std::min(grid, sm_count * calib_resident_blocks<T, KK, BWD, MUL, SEG>()), kCalibBlock, 0, s>>>(         \
             TB, in, (T *)scratch, scratch_bytes_per_warp / (int64_t)sizeof(T), loglik, weights, grad_open,           \
             grad_cont, need_fp64, fp64 ? 1 : 0)
 #define GHMM_CALIB(KK, MUL)                                                                                         \
     if (fp64) {                                                                                                     \
-        if (backward)                                                                                               \
-            GHMM_CALIB_ONE(double, KK, true, MUL);                                                                  \
+        if (backward && seg == kSeg)                                                                                \
+            GHMM_CALIB_ONE(double, KK, true, MUL, kSeg);                                                            \
+        else if (backward)                                                                                          \
+            GHMM_CALIB_ONE(double, KK, true, MUL, kSegLong);                                                        \
         else                                                                                                        \
-            GHMM_CALIB_ONE(double, KK, false, MUL);                                                                 \
+            GHMM_CALIB_ONE(double, KK, false, MUL, kSeg);                                                           \
     } else {                                                                                                        \
-        if (backward)                                                                                               \
-            GHMM_CALIB_ONE(float, KK, true, MUL);                                                                   \
+        if (backward && seg == kSeg)                                                                                \
+            GHMM_CALIB_ONE(float, KK, true, MUL, kSeg);                                                             \
+        else if (backward)                                                                                          \
+            GHMM_CALIB_ONE(float, KK, true, MUL, kSegLong);                                                         \
         else                                                                                                        \
-            GHMM_CALIB_ONE(float, KK, false, MUL);                                                                  \
+            GHMM_CALIB_ONE(float, KK, false, MUL, kSeg);                                                            \
     }
     switch (k) {
         case 1: GHMM_CALIB(1, false) break;

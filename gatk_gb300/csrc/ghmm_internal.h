@@ -183,13 +183,14 @@ int launch_postprocess(const DevBatch &b, int64_t n_reads, const PostArgs &p, ui
                        cudaStream_t s);
 int measure_peaks_device(int sm_count, double *fp32, double *fp32x2, double *fp64, cudaStream_t s);
 // Calibration forward/backward (calib.cu).
-int64_t calib_scratch_per_warp(int k, int max_hap_len, int max_read_len, bool fp64);
+int64_t calib_scratch_per_warp(int k, int max_hap_len, int max_read_len, bool fp64, int seg);
+int calib_seg(int k, int max_hap_len, int max_read_len, int64_t budget, int sm_count);
 constexpr int kCalibMaxRead = 65536;  // calibration reads: one strip up to 256 bases, strips of 256 rows beyond
 int calib_grid(int sm_count);  // blocks of a full grid; a call may launch fewer (scratch budget)
 int calib_block();
 int launch_calib(const DevTables &TB, const ghmm_calib_batch &in, int k, bool backward, bool fp64, void *scratch,
                  int64_t scratch_bytes_per_warp, double *loglik, const double *weights, float *grad_open,
-                 float *grad_cont, int *need_fp64, int grid, int sm_count, cudaStream_t s);
+                 float *grad_cont, int *need_fp64, int seg, int grid, int sm_count, cudaStream_t s);
 int launch_calib_gather(const double *table, int64_t rows, const int64_t *index, int64_t n, double fixed_open,
                         double fixed_cont, float *gap_open, float *gap_cont, int sm_count, cudaStream_t s);
 int launch_calib_fold(const int64_t *index, int64_t n, const float *grad_open, const float *grad_cont, int rows,

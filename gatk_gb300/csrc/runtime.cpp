@@ -238,12 +238,13 @@ static int calib_run(ghmm_ctx *ctx, const ghmm_calib_batch *in, int precision, c
     // the backward keeps checkpoints in per-warp scratch, and a read of several strips passes each strip's last
     // row through it in the forward too
     const bool strips = in->max_read_len > 32 * 8;
-    const int64_t per_warp = calib_scratch_per_warp(k, in->max_hap_len, in->max_read_len, true);  // sized for FP64
+    const int64_t budget = calib_scratch_budget();
+    const int seg = calib_seg(k, in->max_hap_len, in->max_read_len, budget, ctx->sm_count);
+    const int64_t per_warp = calib_scratch_per_warp(k, in->max_hap_len, in->max_read_len, true, seg);  // sized for FP64
     const int64_t warps_per_block = calib_block() / 32;
     int64_t blocks = calib_grid(ctx->sm_count);
     if (backward || strips) {
         // fewer warps (each taking more pairs) where long pairs would make a full grid's scratch exceed the budget
-        const int64_t budget = calib_scratch_budget();
         blocks = std::max<int64_t>(1, std::min(blocks, budget / (per_warp * warps_per_block)));
         GHMM_CUDA(ctx->calib_scratch.reserve((size_t)(per_warp * warps_per_block * blocks)), "calibration scratch");
     }
@@ -264,12 +265,12 @@ static int calib_run(ghmm_ctx *ctx, const ghmm_calib_batch *in, int precision, c
         GHMM_CUDA(cudaStreamSynchronize(s), "H2D flags");
     } else {
         int e = launch_calib(ctx->tables, *in, k, backward, false, ctx->calib_scratch.p,
-                             calib_scratch_per_warp(k, in->max_hap_len, in->max_read_len, false), loglik, weights,
-                             gopen, gcont, flags, (int)blocks, ctx->sm_count, s);
+                             calib_scratch_per_warp(k, in->max_hap_len, in->max_read_len, false, seg), loglik,
+                             weights, gopen, gcont, flags, seg, (int)blocks, ctx->sm_count, s);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "calibration FP32 launch");
     }
     int e = launch_calib(ctx->tables, *in, k, backward, true, ctx->calib_scratch.p, per_warp, loglik, weights, gopen,
-                         gcont, flags, (int)blocks, ctx->sm_count, s);
+                         gcont, flags, seg, (int)blocks, ctx->sm_count, s);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "calibration FP64 launch");
     GHMM_CUDA(cudaStreamSynchronize(s), "calibration kernels");
     return GHMM_OK;

@@ -49,7 +49,8 @@ int ghmm_calib_forward(ghmm_ctx *ctx, const ghmm_calib_batch *batch, int32_t pre
 
 /* Forward and hand-written backward.  d_loglik as above; d_grad_open / d_grad_cont (device, one float per
  * read position, accumulated into, so zero them first) receive sum_p w_p * d log10 L_p / d g (resp. c) with
- * w_p = d_weights[p] (device, NULL: all ones).  The forward is recomputed from checkpoints every 8 wavefront
+ * w_p = d_weights[p] (device, NULL: all ones).  The forward is recomputed from checkpoints every 8 (16 where these would
+ * leave the device short of warps within the scratch limit below) wavefront
  * steps during the backward sweep; reads longer than 256 bases run in strips of 256 rows, whose boundary rows
  * (forward) and first-row adjoints (backward) pass through per-warp scratch, the backward taking the strips last
  * to first.  The context holds that scratch (for the forward too when reads exceed 256 bases): at most
