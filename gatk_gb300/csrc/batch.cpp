@@ -533,10 +533,11 @@ int batch_upload(ghmm_ctx *ctx, ghmm_batch &b, cudaStream_t s) {
     GHMM_CUDA(b.d_nout.reserve(1), "device output count");
     GHMM_CUDA(b.d_scratch32.reserve((size_t)std::max<int64_t>(b.scratch32_size, 1)), "device FP32 strip scratch");
     // columns of the FP64 strip scratch per warp: a haplotype, or a run of them (runs end at what fits)
-    const bool runs64 = b.max_hap_len <= kFp64RunCols && b.max_read_len < kFp64SplitRows;
+    const bool runs64 = b.max_hap_len <= kFp64RunCols;
     const int64_t cols64 = (int64_t)std::max(b.max_hap_len, 1) * (runs64 ? kFp64Run : 1);
     const size_t s64 = (size_t)b.fp64_grid * kWarpsPerBlock * (size_t)cols64 * 3;
     GHMM_CUDA(b.d_scratch64.reserve(s64), "device FP64 strip scratch");
+    if (b.max_read_len >= kFp64SplitRows) GHMM_CUDA(b.d_fp64_long.reserve((size_t)capacity), "device FP64 pair list");
     GHMM_CUDA(b.d_read_scale.reserve((size_t)std::max<int64_t>(NR, 1)), "device read scales");
 
     GHMM_CUDA(cudaMemcpyAsync(b.d_planes.p, b.h_planes.p, (size_t)b.read_bytes * 5, cudaMemcpyHostToDevice, s), "H2D planes");
@@ -672,7 +673,8 @@ int batch_phase(ghmm_ctx *ctx, ghmm_batch &b, int phase, cudaStream_t s) {
         }
         return GHMM_OK;
     }
-    int e = launch_fp64_queue(ctx->tables, b.dev, b.max_read_len >= kFp64SplitRows, b.fp64_grid, s);
+    int32_t *const long_list = b.max_read_len >= kFp64SplitRows ? b.d_fp64_long.p : nullptr;
+    int e = launch_fp64_queue(ctx->tables, b.dev, long_list, b.fp64_grid, ctx->sm_count, s);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "FP64 queue launch");
     return GHMM_OK;
 }
@@ -782,7 +784,7 @@ int batch_enqueue(ghmm_ctx *ctx, ghmm_batch &b, int mode, cudaStream_t s) {
     memcpy(sig.data() + sizeof(DevBatch), &mode, sizeof(int));
     const int has_tasks = b.n_tasks > 0;
     memcpy(sig.data() + sizeof(DevBatch) + sizeof(int), &has_tasks, sizeof(int));
-    const int fp64_args[2] = {b.max_read_len >= kFp64SplitRows, b.fp64_grid};
+    const int64_t fp64_args[2] = {b.max_read_len >= kFp64SplitRows ? (int64_t)(intptr_t)b.d_fp64_long.p : 0, b.fp64_grid};
     sig.insert(sig.end(), (const unsigned char *)fp64_args, (const unsigned char *)fp64_args + sizeof(fp64_args));
     for (auto &bk : b.buckets) {
         const int64_t kg[4] = {bk.key, bk.grid, bk.scratch_begin, bk.scratch_cols};

@@ -353,13 +353,92 @@ __device__ __forceinline__ bool pair_skipped(const DevBatch &B, const Pair64 &P,
     return false;
 }
 
+__device__ __forceinline__ bool long_pair(const DevBatch &B, PairRef pr) {
+    return B.read_off[pr.read + 1] - B.read_off[pr.read] >= kFp64SplitRows;
+}
+
+// Lists the queue's entries of long reads (their indices, in any order), for batches that have such reads.
+template <bool RESCALED>
+__global__ void __launch_bounds__(256) fp64_long_kernel(DevBatch B, int32_t *long_list) {
+    const PairRef *queue = RESCALED ? B.rerun : B.rerun + B.rerun_capacity;
+    const int total = min(B.counters[RESCALED ? 1 : 4], (int)B.rerun_capacity);
+    int *const n_long = &B.counters[kCounterFp64Long + (RESCALED ? 0 : 2)];
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
+        const int i = (int)base + lane;
+        const unsigned found = __ballot_sync(kFull, i < total && long_pair(B, queue[i]));
+        if (!found) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(n_long, __popc(found));
+        at = __shfl_sync(kFull, at, 0);
+        if (found & (1u << lane)) long_list[at + __popc(found & ((1u << lane) - 1u))] = i;
+    }
+}
+
+// The entries of a long list, a pair or run per warp (LONG: but for the long reads'): drawn several at a time while many a
+// warp are left, one by one towards the end.
+template <bool RESCALED, bool LONG>
+__device__ __forceinline__ void pairs_by_warp(const DevTables &T, const DevBatch &B, const PairRef *queue, int total,
+                                              int *cursor, int warps, Run64 &run, double *mine, double *rowM,
+                                              double *rowI, Unit u, int lane) {
+    Strip64<RESCALED> S;
+    double kappa;
+    for (;;) {
+        int t0 = 0, draw = 1;
+        if (lane == 0) {
+            const int left = total - *reinterpret_cast<volatile int *>(cursor);
+            draw = max(1, min(kRun64, left / (2 * warps)));
+            t0 = atomicAdd(cursor, draw);
+        }
+        t0 = __shfl_sync(kFull, t0, 0);
+        draw = __shfl_sync(kFull, draw, 0);
+        if (t0 >= total) break;
+        const int t1 = min(t0 + draw, total);
+        for (int t = t0; t < t1;) {
+            const PairRef pr = queue[t];
+            if (LONG && long_pair(B, pr)) {
+                ++t;
+                continue;
+            }
+            // a run: the same read, the haplotype after the last one's, no empty ones, within the strip scratch
+            int n = 1;
+            const int64_t h0 = B.hap_off[pr.hap];
+            int64_t end = B.hap_off[pr.hap + 1];
+            while (t + n < t1 && end > h0) {
+                const PairRef next = queue[t + n];
+                if (next.read != pr.read || next.hap != pr.hap + n) break;
+                const int64_t e = B.hap_off[next.hap + 1];
+                if (e == end || e - h0 > B.scratch64_cols) break;
+                end = e;
+                ++n;
+            }
+            t += n;
+            Pair64 P = load_pair(B, pr, n);
+            if (pair_skipped(B, P, lane == 0)) continue;
+            pair_scale<RESCALED>(T, B, P, run, kappa, lane);
+            const int strips = (P.blocks32 + 3) / 4, phases = (P.H + 31 + kPhase - 1) / kPhase;
+            Sum64 sum;
+            sum.end = run.end[0];
+            for (int strip = 0; strip < strips; ++strip) {
+                __syncwarp();  // the strip above has written its last row
+                strip_begin<RESCALED>(T, B, P, strip, strips, run.init[0], mine, S, lane);
+                for (int r = 0; r < phases; ++r)
+                    strip_phase<RESCALED>(B, P, run, S, r, mine, mine, rowM, rowI, kappa, sum, u, lane);
+            }
+        }
+    }
+}
+
 // Launched with full grids; queue lengths are device counters, so the choice between a pair per warp and a pair per
 // block is made here.  A pair per block when the list is shorter than the grid's warps (each pair then runs on four
-// sub-partitions) and when the batch has long reads (kFp64SplitRows: a pair's time on one warp, 15 ms at 1,400 x 2,250
-// bases, is what the last pairs of a long list would otherwise take); a pair per warp for long lists of short reads,
-// where the lag of the strips would idle a tenth of the warps.
-template <bool RESCALED>
-__global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables T, DevBatch B, bool long_reads,
+// sub-partitions).  Of longer lists, the pairs of long reads, which go first (LONG, for batches that have such reads:
+// long_list names their entries): a pair's time on one warp, 15 ms at 1,400 x 2,250 bases, is what the last pairs would
+// otherwise take.  A pair per warp for the others: in a block they idle warps in the strips' lag and, having fewer strips
+// than warps, altogether (10,240 pairs of 20, 100 and 250 x 300 bases beside one of 481 x 600: 1.11, 3.74 and 7.42 ms; all
+// of them a pair per block 3.05, 5.57 and 8.98).
+template <bool RESCALED, bool LONG>
+__global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables T, DevBatch B, const int32_t *long_list,
                                                                       Unit u) {
     __shared__ double row_sum[kWarps64][2][kPhase];
     __shared__ Run64 runs[kWarps64];
@@ -372,65 +451,30 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
     double *const mine = block_scratch + (int64_t)warp * B.scratch64_cols * 3;
     double *const rowM = row_sum[warp][0], *const rowI = row_sum[warp][1];
     Run64 &run = runs[warp];
-    Strip64<RESCALED> S;
-    double kappa;
     const int warps = (int)gridDim.x * kWarps64;
-    if (total > warps && !long_reads) {
-        // entries drawn several at a time while many a warp are left, one by one towards the end
-        for (;;) {
-            int t0 = 0, draw = 1;
-            if (lane == 0) {
-                const int left = total - *reinterpret_cast<volatile int *>(cursor);
-                draw = max(1, min(kRun64, left / (2 * warps)));
-                t0 = atomicAdd(cursor, draw);
-            }
-            t0 = __shfl_sync(kFull, t0, 0);
-            draw = __shfl_sync(kFull, draw, 0);
-            if (t0 >= total) break;
-            const int t1 = min(t0 + draw, total);
-            for (int t = t0; t < t1;) {
-                const PairRef pr = queue[t];
-                // a run: the same read, the haplotype after the last one's, no empty ones, within the strip scratch
-                int n = 1;
-                const int64_t h0 = B.hap_off[pr.hap];
-                int64_t end = B.hap_off[pr.hap + 1];
-                while (t + n < t1 && end > h0) {
-                    const PairRef next = queue[t + n];
-                    if (next.read != pr.read || next.hap != pr.hap + n) break;
-                    const int64_t e = B.hap_off[next.hap + 1];
-                    if (e == end || e - h0 > B.scratch64_cols) break;
-                    end = e;
-                    ++n;
-                }
-                t += n;
-                Pair64 P = load_pair(B, pr, n);
-                if (pair_skipped(B, P, lane == 0)) continue;
-                pair_scale<RESCALED>(T, B, P, run, kappa, lane);
-                const int strips = (P.blocks32 + 3) / 4, phases = (P.H + 31 + kPhase - 1) / kPhase;
-                Sum64 sum;
-                sum.end = run.end[0];
-                for (int strip = 0; strip < strips; ++strip) {
-                    __syncwarp();  // the strip above has written its last row
-                    strip_begin<RESCALED>(T, B, P, strip, strips, run.init[0], mine, S, lane);
-                    for (int r = 0; r < phases; ++r)
-                        strip_phase<RESCALED>(B, P, run, S, r, mine, mine, rowM, rowI, kappa, sum, u, lane);
-                }
-            }
-        }
+    if (!LONG && total > warps) {
+        pairs_by_warp<RESCALED, LONG>(T, B, queue, total, cursor, warps, run, mine, rowM, rowI, u, lane);
         return;
     }
+    // a pair per block: the whole queue, or of a long one the listed entries
+    Strip64<RESCALED> S;
+    double kappa;
+    const bool listed = LONG && total > warps;
+    int *const counters = &B.counters[kCounterFp64Long + (RESCALED ? 0 : 2)];
+    const int n_pairs = listed ? counters[0] : total;
+    int *const next_pair = listed ? counters + 1 : cursor;
     const double *const above = block_scratch + (int64_t)((warp + kWarps64 - 1) % kWarps64) * B.scratch64_cols * 3;
     for (bool first = true;;) {
         int t = blockIdx.x;
         if (!first) {
             __syncthreads();  // every warp has read the previous job
-            if (threadIdx.x == 0) job = (int)gridDim.x + atomicAdd(cursor, 1);
+            if (threadIdx.x == 0) job = (int)gridDim.x + atomicAdd(next_pair, 1);
             __syncthreads();
             t = job;
         }
         first = false;
-        if (t >= total) break;
-        Pair64 P = load_pair(B, queue[t]);
+        if (t >= n_pairs) break;
+        Pair64 P = load_pair(B, queue[listed ? long_list[t] : t]);
         if (pair_skipped(B, P, threadIdx.x == 0)) continue;
         pair_scale<RESCALED>(T, B, P, run, kappa, lane);
         // strips of at most 128 rows, a multiple of four of them where the rows allow; strip s runs on warp s % 4 from
@@ -455,26 +499,36 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
             __syncthreads();
         }
     }
+    if (listed) pairs_by_warp<RESCALED, LONG>(T, B, queue, total, cursor, warps, run, mine, rowM, rowI, u, lane);
 }
 
 }  // namespace
 
-int launch_fp64_queue(const DevTables &t, const DevBatch &b, bool long_reads, int grid, cudaStream_t s) {
+int launch_fp64_queue(const DevTables &t, const DevBatch &b, int32_t *long_list, int grid, int sm_count, cudaStream_t s) {
     const Unit u{0.0, 1.0};
-    fp64_queue_kernel<true><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_reads, u);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    fp64_queue_kernel<false><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_reads, u);
+    if (long_list) {
+        fp64_long_kernel<true><<<sm_count, 256, 0, s>>>(b, long_list);
+        fp64_queue_kernel<true, true><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_list, u);
+        fp64_long_kernel<false><<<sm_count, 256, 0, s>>>(b, long_list);
+        fp64_queue_kernel<false, true><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_list, u);
+    } else {
+        fp64_queue_kernel<true, false><<<grid, 32 * kWarps64, 0, s>>>(t, b, nullptr, u);
+        fp64_queue_kernel<false, false><<<grid, 32 * kWarps64, 0, s>>>(t, b, nullptr, u);
+    }
     return (int)cudaGetLastError();
 }
 
 int fp64_kernel_occupancy(int *blocks_per_sm) {
-    // both tiers run on the same grid and scratch: the smaller occupancy of the two
-    int a = 0, b = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fp64_queue_kernel<true>, 32 * kWarps64, 0);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fp64_queue_kernel<false>, 32 * kWarps64, 0);
-    *blocks_per_sm = a < b ? a : b;
+    // both tiers run on the same grid and scratch: the smallest occupancy of the forms
+    const void *fns[] = {(const void *)fp64_queue_kernel<true, false>, (const void *)fp64_queue_kernel<false, false>,
+                         (const void *)fp64_queue_kernel<true, true>, (const void *)fp64_queue_kernel<false, true>};
+    cudaError_t e = cudaSuccess;
+    *blocks_per_sm = INT32_MAX;
+    for (const void *fn : fns) {
+        int n = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, 32 * kWarps64, 0);
+        *blocks_per_sm = n < *blocks_per_sm ? n : *blocks_per_sm;
+    }
     return (int)e;
 }
 

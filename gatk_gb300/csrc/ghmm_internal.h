@@ -92,10 +92,12 @@ struct DevBatch {
 
 // Kernel launchers (kernels.cu).  All return cudaError_t as int.
 int launch_fp32_bucket(const DevTables &t, const DevBatch &b, int key, int grid, int block, cudaStream_t s);
-int launch_fp64_queue(const DevTables &t, const DevBatch &b, bool long_reads, int grid, cudaStream_t s);  // fp64.cu
+// The FP64 queues (fp64.cu); long_list: rerun_capacity indices of scratch where the batch has long reads, else null.
+int launch_fp64_queue(const DevTables &t, const DevBatch &b, int32_t *long_list, int grid, int sm_count, cudaStream_t s);
 constexpr int kFp64Run = 4;          // haplotypes of one read a warp may take as one stream ...
 constexpr int kFp64RunCols = 2048;   // ... in batches whose haplotypes are all of up to this many columns
-constexpr int kFp64SplitRows = 481;  // batches with reads of this many bases run a pair per block at any queue length
+constexpr int kFp64SplitRows = 481;  // reads of this many bases run a pair per block at any queue length (fp64.cu)
+constexpr int kCounterFp64Long = 40;  // counters[40]: long reads' pairs in queue 1, [41] their cursor; [42], [43]: queue 2's
 int launch_finalize_fp32(double *out, const int64_t *n_out, int sm_count, cudaStream_t s);
 // Per-read log2 a_R of the FP32 pass (kernels.cu), into scale[n_reads]; after the read planes are final.
 int launch_read_scale(const DevTables &t, const DevBatch &b, int64_t n_reads, float2 *scale, int sm_count,

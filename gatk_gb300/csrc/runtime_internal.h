@@ -105,6 +105,7 @@ struct ghmm_batch {
     bool has_pd = false;
     PdPlanes pd{};
     DevBuf<float4> d_scratch32;
+    DevBuf<int32_t> d_fp64_long;  // (of batches with long reads)
     DevBuf<double> d_scratch64;
     DevBuf<float2> d_read_scale;  // per read: the FP32 pass's log2 a_R as (2^-(la - n), n), from launch_read_scale
     // sizes
@@ -147,7 +148,7 @@ struct ghmm_batch {
         auto add = [&n](const auto &...buf) { ((n += buf.cap * sizeof(*buf.p)), ...); };
         add(h_planes, h_hap, h_off, h_read_region, h_init_f, h_init_d, h_tasks, h_direct, h_fp64all, h_out, h_counters,
             h_nout, d_planes, d_hap, d_off, d_read_region, d_init_f, d_init_d, d_tasks, d_rerun, d_out, d_counters, d_nout,
-            d_post, h_mapq, d_mapq, h_dragstr, d_dragstr, h_pd, d_pd, d_scratch32, d_scratch64, d_read_scale);
+            d_post, h_mapq, d_mapq, h_dragstr, d_dragstr, h_pd, d_pd, d_scratch32, d_scratch64, d_read_scale, d_fp64_long);
         return n;
     }
 
@@ -183,7 +184,7 @@ struct ghmm_batch {
         h_init_d.release(); h_tasks.release(); h_direct.release(); h_fp64all.release(); h_out.release(); h_counters.release();
         d_planes.release(); d_hap.release(); d_off.release(); d_read_region.release(); d_init_f.release();
         d_init_d.release(); d_tasks.release(); d_rerun.release(); d_out.release(); d_counters.release();
-        d_scratch32.release(); d_scratch64.release(); d_read_scale.release(); d_post.release(); h_pd.release();
+        d_fp64_long.release(); d_scratch32.release(); d_scratch64.release(); d_read_scale.release(); d_post.release(); h_pd.release();
         d_pd.release();
         h_mapq.release(); d_mapq.release(); h_dragstr.release(); d_dragstr.release();
         has_pd = false;
