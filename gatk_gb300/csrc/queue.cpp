@@ -12,6 +12,7 @@
 #include <deque>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <numeric>
 #include <string>
 #include <thread>
@@ -422,7 +423,8 @@ int pipelined_compute(ghmm_ctx *ctx, const Source &src, const std::vector<int64_
     const int64_t hold = reg_out[(size_t)cut[cut.size() - 2]];  // results of all units but the last
     if (hold > q->held_cap) {
         q->held_cap = 0;
-        q->held.reset(new double[(size_t)hold]);
+        q->held.reset(new (std::nothrow) double[(size_t)hold]);
+        if (!q->held) return fail(ctx, GHMM_ERR_NOMEM, "results of a call's batches");
         q->held_cap = hold;
     }
     for (size_t i = 0; i + 1 < cut.size(); i++) {
@@ -508,14 +510,23 @@ int compute_sync(ghmm_ctx *ctx, const Source &src, double *out) {
 
 extern "C" {
 
-int ghmm_debug_pipeline_cuts(const int64_t *cells, int64_t n_regions, int64_t *cuts, int64_t cap, int64_t *n_cuts) {
+static int debug_cuts(std::vector<int64_t> (*rule)(const std::vector<int64_t> &), const int64_t *cells, int64_t n_regions,
+                      int64_t *cuts, int64_t cap, int64_t *n_cuts) {
     if (n_regions < 0 || (n_regions > 0 && !cells) || cap < 0 || (cap > 0 && !cuts) || !n_cuts) return GHMM_ERR_ARG;
     for (int64_t g = 0; g < n_regions; g++)
         if (cells[g] < 0) return GHMM_ERR_ARG;
-    const std::vector<int64_t> cut = pipeline_cuts(std::vector<int64_t>(cells, cells + n_regions));
+    const std::vector<int64_t> cut = rule(std::vector<int64_t>(cells, cells + n_regions));
     *n_cuts = (int64_t)cut.size();
     for (int64_t i = 0; i < std::min<int64_t>(cap, (int64_t)cut.size()); i++) cuts[i] = cut[(size_t)i];
     return GHMM_OK;
+}
+
+int ghmm_debug_pipeline_cuts(const int64_t *cells, int64_t n_regions, int64_t *cuts, int64_t cap, int64_t *n_cuts) {
+    return debug_cuts(pipeline_cuts, cells, n_regions, cuts, cap, n_cuts);
+}
+
+int ghmm_debug_call_cuts(const int64_t *cells, int64_t n_regions, int64_t *cuts, int64_t cap, int64_t *n_cuts) {
+    return debug_cuts(call_cuts, cells, n_regions, cuts, cap, n_cuts);
 }
 
 int ghmm_queue_create(ghmm_ctx *ctx, int64_t batch_cells, ghmm_queue **queue) {

@@ -420,6 +420,10 @@ int ghmm_debug_pd_ops(const uint8_t *bases, const uint8_t *pd_flags, int32_t H, 
  * cell number or a NULL array. */
 int ghmm_debug_pipeline_cuts(const int64_t *cells, int64_t n_regions, int64_t *cuts, int64_t cap, int64_t *n_cuts);
 
+/* The same for a regular call that runs as a pipeline (ghmm_compute_regions): the first chunk takes 1/8 of the cells, at
+ * most 8e9, each next one 2.5 times the last, up to 1/3 of all. */
+int ghmm_debug_call_cuts(const int64_t *cells, int64_t n_regions, int64_t *cuts, int64_t cap, int64_t *n_cuts);
+
 /* ---- Several devices from one caller ----
  * One handle drives several GPUs (HaplotypeCaller's one JVM; the reference parallelises the host side with GKL's
  * thread count, HC/PairHMMNativeArgumentCollection.java:11-12, or one engine per Spark partition,
