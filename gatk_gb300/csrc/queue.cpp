@@ -26,7 +26,9 @@ namespace rt {
 
 constexpr size_t kQueueMaxReady = 2;  // sealed batches waiting for the worker before push blocks
 
-// The results of unit u as blocks of at most 1M, in parallel: f(source, destination, index within the unit, count).
+// The results of unit u as blocks of at most 64K, in parallel: f(source, destination, index within the unit, count).
+// (A caller's new array has its pages made here: 8 MB blocks left most cores idle over the 48 MB that a call of 6,000
+// regions delivers while its last large batch runs: 155.8 ms a call, with these 153.8.)
 template <typename F>
 void for_result_blocks(const QueueUnit &u, const double *src, int threads, F f) {
     struct Block {
@@ -34,10 +36,11 @@ void for_result_blocks(const QueueUnit &u, const double *src, int threads, F f) 
         int64_t at, n;
     };
     std::vector<Block> blocks;
+    constexpr int64_t kBlockResults = 1 << 16;
     int64_t base = 0;
     for (const auto &d : u.dests) {
-        for (int64_t a = 0; a < d.second; a += (1 << 20))
-            blocks.push_back(Block{d.first + a, base + a, std::min<int64_t>(d.second - a, 1 << 20)});
+        for (int64_t a = 0; a < d.second; a += kBlockResults)
+            blocks.push_back(Block{d.first + a, base + a, std::min(d.second - a, kBlockResults)});
         base += d.second;
     }
     parallel_for((int64_t)blocks.size(), threads, [&](int64_t k) {
