@@ -357,23 +357,36 @@ __device__ __forceinline__ bool long_pair(const DevBatch &B, PairRef pr) {
     return B.read_off[pr.read + 1] - B.read_off[pr.read] >= kFp64SplitRows;
 }
 
-// Lists the queue's entries of long reads (their indices, in any order), for batches that have such reads.
+// Lists the queue's entries of long reads (their indices, in the queue's order), for batches that have such reads: each
+// block those of its part of the queue, behind those that it counts in the parts before (half a millisecond for a million
+// entries).  In any order that atomics give, 5,172 pairs of 800-2,000 bases took 161 ms instead of 158.
+constexpr int kListThreads = 1024;
 template <bool RESCALED>
-__global__ void __launch_bounds__(256) fp64_long_kernel(DevBatch B, int32_t *long_list) {
+__global__ void __launch_bounds__(kListThreads) fp64_long_kernel(DevBatch B, int32_t *long_list) {
+    __shared__ int warp_count[kListThreads / 32];
     const PairRef *queue = RESCALED ? B.rerun : B.rerun + B.rerun_capacity;
     const int total = min(B.counters[RESCALED ? 1 : 4], (int)B.rerun_capacity);
-    int *const n_long = &B.counters[kCounterFp64Long + (RESCALED ? 0 : 2)];
-    const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-        const int i = (int)base + lane;
-        const unsigned found = __ballot_sync(kFull, i < total && long_pair(B, queue[i]));
-        if (!found) continue;
-        int at = 0;
-        if (lane == 0) at = atomicAdd(n_long, __popc(found));
-        at = __shfl_sync(kFull, at, 0);
-        if (found & (1u << lane)) long_list[at + __popc(found & ((1u << lane) - 1u))] = i;
+    const int begin = (int)((int64_t)total * blockIdx.x / gridDim.x);
+    const int end = (int)((int64_t)total * (blockIdx.x + 1) / gridDim.x);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int at = 0;
+    for (int base = 0; base < begin; base += kListThreads) {
+        const int i = base + (int)threadIdx.x;
+        at += __syncthreads_count(i < begin && long_pair(B, queue[i]));
     }
+    for (int base = begin; base < end; base += kListThreads) {
+        const int i = base + (int)threadIdx.x;
+        const bool found = i < end && long_pair(B, queue[i]);
+        const unsigned mine = __ballot_sync(kFull, found);
+        if (lane == 0) warp_count[warp] = __popc(mine);
+        const int here = __syncthreads_count(found);
+        int slot = at + __popc(mine & ((1u << lane) - 1u));
+        for (int w = 0; w < warp; ++w) slot += warp_count[w];
+        if (found) long_list[slot] = i;
+        at += here;
+        __syncthreads();  // every warp has read the counts
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) B.counters[kCounterFp64Long + (RESCALED ? 0 : 2)] = at;
 }
 
 // The entries of a long list, a pair or run per warp (LONG: but for the long reads'): drawn several at a time while many a
@@ -381,9 +394,8 @@ __global__ void __launch_bounds__(256) fp64_long_kernel(DevBatch B, int32_t *lon
 template <bool RESCALED, bool LONG>
 __device__ __forceinline__ void pairs_by_warp(const DevTables &T, const DevBatch &B, const PairRef *queue, int total,
                                               int *cursor, int warps, Run64 &run, double *mine, double *rowM,
-                                              double *rowI, Unit u, int lane) {
-    Strip64<RESCALED> S;
-    double kappa;
+                                              double *rowI, Unit u, int lane,
+                                              Strip64<RESCALED> &S, double &kappa) {
     for (;;) {
         int t0 = 0, draw = 1;
         if (lane == 0) {
@@ -451,14 +463,14 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
     double *const mine = block_scratch + (int64_t)warp * B.scratch64_cols * 3;
     double *const rowM = row_sum[warp][0], *const rowI = row_sum[warp][1];
     Run64 &run = runs[warp];
+    Strip64<RESCALED> S;
+    double kappa;
     const int warps = (int)gridDim.x * kWarps64;
     if (!LONG && total > warps) {
-        pairs_by_warp<RESCALED, LONG>(T, B, queue, total, cursor, warps, run, mine, rowM, rowI, u, lane);
+        pairs_by_warp<RESCALED, LONG>(T, B, queue, total, cursor, warps, run, mine, rowM, rowI, u, lane, S, kappa);
         return;
     }
     // a pair per block: the whole queue, or of a long one the listed entries
-    Strip64<RESCALED> S;
-    double kappa;
     const bool listed = LONG && total > warps;
     int *const counters = &B.counters[kCounterFp64Long + (RESCALED ? 0 : 2)];
     const int n_pairs = listed ? counters[0] : total;
@@ -499,7 +511,7 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
             __syncthreads();
         }
     }
-    if (listed) pairs_by_warp<RESCALED, LONG>(T, B, queue, total, cursor, warps, run, mine, rowM, rowI, u, lane);
+    if (listed) pairs_by_warp<RESCALED, LONG>(T, B, queue, total, cursor, warps, run, mine, rowM, rowI, u, lane, S, kappa);
 }
 
 }  // namespace
@@ -507,9 +519,9 @@ __global__ void __launch_bounds__(32 * kWarps64, 3) fp64_queue_kernel(DevTables 
 int launch_fp64_queue(const DevTables &t, const DevBatch &b, int32_t *long_list, int grid, int sm_count, cudaStream_t s) {
     const Unit u{0.0, 1.0};
     if (long_list) {
-        fp64_long_kernel<true><<<sm_count, 256, 0, s>>>(b, long_list);
+        fp64_long_kernel<true><<<sm_count, kListThreads, 0, s>>>(b, long_list);
         fp64_queue_kernel<true, true><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_list, u);
-        fp64_long_kernel<false><<<sm_count, 256, 0, s>>>(b, long_list);
+        fp64_long_kernel<false><<<sm_count, kListThreads, 0, s>>>(b, long_list);
         fp64_queue_kernel<false, true><<<grid, 32 * kWarps64, 0, s>>>(t, b, long_list, u);
     } else {
         fp64_queue_kernel<true, false><<<grid, 32 * kWarps64, 0, s>>>(t, b, nullptr, u);
