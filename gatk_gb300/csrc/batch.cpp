@@ -115,9 +115,10 @@ int plan_sizes(ghmm_ctx *ctx, const Source &src, ghmm_batch &b, std::vector<int6
 
 
 // Haplotype columns per FP32 task for a batch whose read pairs meet pair_cols columns in all (strips counted apart),
-// at most max_cols (the tuning's chunk_cols).  A large batch has many tasks per warp slot (12 a SM) and takes max_cols;
-// a small one would leave most slots empty and end in the time of its longest task, so its regions are cut until
-// a slot gets about four tasks, down to one haplotype each.  Each cut costs the wavefront's fill (62 steps) and the
+// at most max_cols (the tuning's chunk_cols).  A large batch has many tasks per warp slot and takes max_cols; a small one
+// would leave most slots empty and end in the time of its longest task, so its regions are cut until a slot gets about four
+// tasks, down to one haplotype each.  Slots are counted as the 12 an SM of buckets of six rows per lane and more; those of
+// fewer rows have 16, and then get about three tasks each.  Each cut costs the wavefront's fill (62 steps) and the
 // row coefficients once more: about 2 % of a task at the 3,900 columns that a region of 2,000 reads x 64 haplotypes
 // gets.  Whole calls, with the buckets side by side (fork_buckets) in both: that region 9.2 -> 6.2 ms; 600 reads of
 // 260-600 bases x 24 haplotypes of 800 38.0 -> 10.9 ms; 600 regions (16,384 columns before and after) 19.1 -> 17.5 ms

@@ -82,11 +82,10 @@ struct DevBatch {
     const int64_t *n_out_dev;   // number of outputs (for the FP64 epilogue)
     int64_t rerun_capacity;
     int64_t force_rerun_every;  // test hook (ghmm_debug_inject): every n-th output of the FP32 pass goes to FP64; 0 off
-    // strip-boundary scratch of multi-strip FP32 tasks: per resident warp, max_cols float2 x 3
     float4 *scratch32;       // strip boundary: per warp and column a lane's hand-over, (I~, M~ inner sum) of both reads
     int64_t scratch32_cols;  // columns a warp, of the bucket being launched (fork_buckets)
-    double *scratch64;          // FP64 multi-strip boundary: per resident warp, max_hap_len x 3 doubles
-    int64_t scratch64_cols;
+    double *scratch64;          // FP64 strip boundary: per resident warp, scratch64_cols x 3 doubles (PD-HMM: x 6)
+    int64_t scratch64_cols;     // the longest haplotype's columns, or what a run of haplotypes may have (batch_upload)
     const float2 *read_scale;   // per read: (2^-(la - n), n) with la = log2 a_R of the FP32 pass, n = round(la)
 };
 

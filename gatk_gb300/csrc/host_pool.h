@@ -1,5 +1,6 @@
 // host_pool.h -- the worker threads that the host loops of a process's contexts share.  Starting threads for every
-// loop cost about 0.13 ms a thread on the GB300 hosts' Arm cores: 2 ms of a 2.0 ms one-region call.
+// loop cost about 0.13 ms a thread on the GB300 hosts' Arm cores: a call of one region, with three loops, took 2.0 ms,
+// with the pool 0.43.
 #pragma once
 
 #include <condition_variable>

@@ -329,9 +329,9 @@ struct RawView {
     RouteBound bound;
 };
 
-// runtime.cpp: status and message of a failed call (into the queue worker's own message on its thread)
 // runtime.cpp: a batch for a new handle, with the buffers of the context's last destroyed one where it kept them
 ghmm_batch *new_batch(ghmm_ctx *ctx);
+// runtime.cpp: status and message of a failed call (into the queue worker's own message on its thread)
 extern thread_local std::string *t_error_sink;
 int fail(ghmm_ctx *ctx, int code, const std::string &msg);
 int cuda_fail(ghmm_ctx *ctx, cudaError_t e, const char *what);

@@ -10,7 +10,8 @@ namespace {
 // warp w + 1 of any, the following ones from an atomic cursor.  A list shorter than the grid then spreads over all SM
 // sub-partitions; drawn by the cursor alone it goes to whichever blocks start first, up to three warps on one
 // sub-partition while others stand idle, which for FP64 work (one FP64 pipe a sub-partition) costs as many times
-// (615 FP64 reruns of 300 PD-HMM regions: 2.8 ms, spread 1.5 ms).
+// (the FP64 PD-HMM kernel on 100 pairs of 250 x 300 bases: 3.57 ms, spread 1.72; on 600 3.65 and 1.89; on 10,000, more
+// than the grid has warps, 20.4 both ways).
 __device__ __forceinline__ int draw_entry(int *cursor, bool &first, int lane) {
     if (first) {
         first = false;
