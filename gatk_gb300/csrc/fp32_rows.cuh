@@ -1,5 +1,5 @@
 // fp32_rows.cuh -- row coefficients and packed-float helpers shared by the FP32 wavefront kernels
-// (fp32_bucket_kernel in kernels.cu, pd_bucket_kernel in pd_packed.cu).  Internal linkage: each translation unit
+// (fp32_bucket_kernel in fp32_bucket.cuh, pd_bucket_kernel in pd_packed.cu).  Internal linkage: each translation unit
 // that includes it gets its own copy.
 #pragma once
 #include <cuda_runtime.h>

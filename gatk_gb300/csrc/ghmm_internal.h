@@ -113,6 +113,8 @@ constexpr int kCodePad = 64;
 // worst case, and a pair whose rescaled states do overflow sums to a non-finite value and moves to the exact tier, so
 // this only keeps pairs that would almost surely overflow from running twice).
 constexpr double kMaxGrowth64 = 1e15;
+int launch_fp32_mixed(const DevTables &t, const DevBatch &b, int key, int grid, int block, cudaStream_t s);  // fp32_mixed.cu
+int fp32_mixed_occupancy(int key, int block, int *blocks_per_sm);
 int fp32_kernel_occupancy(int key, int block, int *blocks_per_sm);
 int fp64_kernel_occupancy(int *blocks_per_sm);
 

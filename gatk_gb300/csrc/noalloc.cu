@@ -5,7 +5,7 @@
 // caller that cannot take the implicit synchronisation an allocation brings.  ghmm_forward_pairs_noalloc
 // serves them: it computes log10 likelihoods of explicit (read, haplotype) pairs whose bytes the caller
 // already holds in device memory, writes them to a device array the caller provides, and allocates
-// nothing.  The kernel is a variant of the FP64 wavefront kernel (kernels.cu): one pair per warp, four
+// nothing.  The kernel is a variant of the FP64 wavefront kernel (fp64.cu): one pair per warp, four
 // rows per lane, strips of 128 rows for longer reads.  Its strip-boundary scratch and its Phred lookup
 // tables live in the file-scope static __device__ arrays below, which every GPU that loads the library
 // holds until the process exits (12 MiB of scratch plus 134 KiB of tables).

@@ -14,7 +14,7 @@
 // The prior also matches a read base against an undetermined SNP's alternative (isBasePDMatching, :196-210).
 //
 // Kernel: one (read, haplotype) pair per warp, K rows per lane (K = 1..4, per read the strip height that wastes the
-// fewest padding rows), the anti-diagonal wavefront of the FP64 kernels in kernels.cu with six values per row,
+// fewest padding rows), the anti-diagonal wavefront of the FP64 kernels (fp64.cu) with six values per row,
 // strips of 32*K rows through per-warp scratch (six values per column).  Steps where no lane of the warp is at an
 // AFTER_DEL or DEL_END column (nearly all) take a path without max(); the rest take the general one.  Two precisions
 // of the same code:

@@ -9,7 +9,7 @@
 // and at a DEL_END column I reads max(bX, X) of the row above.  An undetermined SNP column also matches a read
 // base against its alternative (isBasePDMatching, :196-210).
 //
-// pd_bucket_kernel<K> runs these pairs as the regular FP32 pass does (fp32_bucket_kernel in kernels.cu, whose
+// pd_bucket_kernel<K> runs these pairs as the regular FP32 pass does (fp32_bucket_kernel in fp32_bucket.cuh, whose
 // header comment describes the layout): read-pair tasks of two reads of one region in the halves of float2, K rows
 // per lane, the region's haplotypes streamed back to back, the two-column lane skew with its hand-over of row 0's
 // I~ and M~ inner sum, rescaled rows, the per-warp prior table and the accumulator rows.  Rescaling a row by a
